@@ -207,3 +207,99 @@ def tolerance(case):
     if case["kind"] == "eval":
         return {"rel": 0.002, "max": 0.01}
     return {"rel": 0.03, "max": 0.9}
+
+
+# ---------------------------------------------------------------------------------------------
+# the same results in 64 bits, in plain torch
+# ---------------------------------------------------------------------------------------------
+def _norm64(x, w, b):
+    return torch.nn.functional.layer_norm(x, (x.shape[-1],), w, b, 1e-5)
+
+
+def _attention64(q, k, v, heads):
+    T, C = q.shape
+    q, k, v = (t.view(T, heads, C // heads).transpose(0, 1) for t in (q, k, v))
+    scores = (q @ k.transpose(1, 2)) / math.sqrt(C // heads)
+    scores = scores.masked_fill(torch.ones(T, T, dtype=torch.bool, device=q.device).triu(1), -math.inf)
+    return (scores.softmax(-1) @ v).transpose(0, 1).reshape(T, C)
+
+
+def _logits64(case, p, x):
+    """Logits [T, V] of one sequence of tokens; `p` holds 64-bit parameters by name."""
+    linear, heads = torch.nn.functional.linear, case["heads"]
+    if case["kind"] == "char":
+        h = p["tok_to_emb.weight"][x] + p["pos_to_emb.weight"][:len(x)]
+        for i in range(case["layers"]):
+            b = f"blocks.{i}."
+            n = _norm64(h, p[b + "ln1.weight"], p[b + "ln1.bias"])
+            q, k, v = (torch.cat([linear(n, p[f"{b}attn.heads.{j}.{which}.weight"]) for j in range(heads)], -1)
+                       for which in ("query", "key", "value"))
+            h = h + linear(_attention64(q, k, v, heads), p[b + "attn.proj.weight"], p[b + "attn.proj.bias"])
+            n = _norm64(h, p[b + "ln2.weight"], p[b + "ln2.bias"])
+            n = linear(n, p[b + "ff.ff.0.weight"], p[b + "ff.ff.0.bias"]).relu()
+            h = h + linear(n, p[b + "ff.ff.3.weight"], p[b + "ff.ff.3.bias"])
+        return linear(_norm64(h, p["ln.weight"], p["ln.bias"]), p["head.weight"], p["head.bias"])
+    h = p["transformer.wte.weight"][x] + p["transformer.wpe.weight"][:len(x)]
+    for i in range(case["layers"]):
+        b = f"transformer.h.{i}."
+        n = _norm64(h, p[b + "ln_1.weight"], p.get(b + "ln_1.bias"))
+        q, k, v = linear(n, p[b + "attn.c_attn.weight"], p[b + "attn.c_attn.bias"]).chunk(3, -1)
+        h = h + linear(_attention64(q, k, v, heads), p[b + "attn.c_proj.weight"], p[b + "attn.c_proj.bias"])
+        n = _norm64(h, p[b + "ln_2.weight"], p.get(b + "ln_2.bias"))
+        n = linear(n, p[b + "mlp.c_fc.weight"], p[b + "mlp.c_fc.bias"])
+        n = torch.nn.functional.gelu(n, approximate="tanh")
+        h = h + linear(n, p[b + "mlp.c_proj.weight"], p[b + "mlp.c_proj.bias"])
+    h = _norm64(h, p["transformer.ln_f.weight"], p.get("transformer.ln_f.bias"))
+    return linear(h, p["transformer.wte.weight"])
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "generate" or case.get("dropout", 0.0) > 0.0 or work(case)["flops"] > 1.2e14:
+        return None  # tokens of its own, a mask that is this framework's own, or too long in 64 bits
+    state = prepare(case, seed)
+    if kind in ("train", "eval"):
+        eng = state["engine"]
+        p = {n: v.double() for n, v in eng.state_dict().items() if n != "lm_head.weight"}
+        batches = [(x.cuda(), y.cuda()) for x, y in state["batches"]]
+    else:
+        p = {n: v.detach().double() for n, v in state["model"].named_parameters()}
+        batches = [(state["X"], state["Y"])]
+    grad = kind != "eval"
+    for v in p.values():
+        v.requires_grad_(grad)
+    tokens = sum(x.numel() for x, _ in batches)
+    per_token, logits, loss = [], [], 0.0
+    with torch.set_grad_enabled(grad):
+        for X, Y in batches:
+            for x, y in zip(X, Y):
+                z = _logits64(case, p, x)
+                ce = torch.nn.functional.cross_entropy(z, y, reduction="none")
+                if grad:
+                    (ce.sum() / tokens).backward()
+                per_token.append(ce.detach())
+                loss += ce.detach().sum() / tokens
+                if kind in ("module", "char"):
+                    logits.append(z.detach())
+    if kind == "eval":
+        return torch.stack(per_token)
+    if kind != "train":
+        flat = torch.nn.utils.parameters_to_vector
+        return {"logits": torch.stack(logits), "loss": loss,
+                "matrix_grads": flat(v.grad for v in p.values() if v.dim() >= 2),
+                "vector_grads": flat(v.grad for v in p.values() if v.dim() < 2)}
+    # first AdamW step, in the order of the engine's flat buffers (gaps between tensors stay 0)
+    oc, k = eng.cfg.optim, eng.layout.n_decay
+    norm = torch.sqrt(sum(v.grad.square().sum() for v in p.values()))
+    clip = min(1.0, oc.clip_norm / (norm.item() + 1e-6))
+    lr = oc.lr_max / oc.warmup_steps
+    w, m, s = (torch.zeros(eng.layout.total, dtype=torch.float64, device="cuda") for _ in range(3))
+    for name, spec in eng.layout.specs.items():
+        at, v = slice(spec.offset, spec.offset + spec.numel), p[name]
+        g = clip * v.grad.flatten()
+        m[at], s[at] = (1 - oc.beta1) * g, (1 - oc.beta2) * g * g
+        step = lr * g / (g.abs() + oc.eps)
+        w[at] = v.detach().flatten() * (1 - lr * oc.weight_decay if spec.decay else 1.0) - step
+    return {"loss": loss, "grad_norm": norm.reshape(1),
+            "matrices": {"weights": w[:k], "m": m[:k], "v": s[:k]},
+            "vectors": {"weights": w[k:], "m": m[k:], "v": s[k:]}}
