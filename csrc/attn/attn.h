@@ -34,4 +34,10 @@ int flash_bwd_ex(const void* qkv, const void* out, const void* dout, const float
                  float* dq_accum, float* stats, int B, int T, int H, float drop_p,
                  const unsigned long long* seed_ptr, unsigned int site, float* dbias, int ordered, int* status,
                  cudaStream_t stream);
+// The same with `dq_copies` times the dq_accum scratch: with a copy for each of the ceil(T / 128) KV tiles
+// the ordered form is one launch whose tiles store to copies of their own (same bits).
+int flash_bwd_sliced(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv,
+                     float* dq_accum, float* stats, int B, int T, int H, float drop_p,
+                     const unsigned long long* seed_ptr, unsigned int site, float* dbias, int ordered, int dq_copies,
+                     int* status, cudaStream_t stream);
 }  // namespace z2h

@@ -40,3 +40,33 @@ def test_layernorm_backward(M, C, bias, extra):
     again = torch.empty_like(x)
     N.layernorm_bwd(dy, x, w, mean, rstd, res if extra else None, again, dw, db, scratch, dxsum=dxsum)
     assert torch.equal(again, dx)
+
+
+# one tile, a second one of one row, several tiles and sequences whose rows share 32-row blocks
+@pytest.mark.parametrize("B,T,H,p", [(1, 128, 1, 0.0), (2, 129, 2, 0.0), (3, 509, 2, 0.0), (2, 1024, 1, 0.2)])
+def test_ordered_attention_backward_in_one_launch(B, T, H, p):
+    from zero_to_hero_b200.ops import native as N
+
+    C = 64 * H
+    g = torch.Generator().manual_seed(T)
+    qkv = (0.7 * torch.randn(B * T, 3 * C, generator=g)).bfloat16().cuda()
+    out, dout = torch.empty(B * T, C, device="cuda", dtype=torch.bfloat16), torch.randn(B * T, C, generator=g).bfloat16().cuda()
+    lse = torch.empty(B, H, T, device="cuda")
+    seed = torch.tensor([3], device="cuda")
+    N.flash_fwd(qkv, out, lse, B, T, H, p, seed, 1)
+    elems, results = N.flash_bwd_dq_elems(B, T, H), []
+    copies = N.flash_bwd_copies(B, T, H)
+    assert copies == (T + 127) // 128
+    for n in (1, copies, copies):  # a launch per KV tile, then one launch, twice
+        dqkv = torch.zeros_like(qkv)
+        dq = torch.full((n * elems,), float("nan"), device="cuda")
+        N.flash_bwd(qkv, out, dout, lse, dqkv, dq, torch.empty(N.flash_bwd_stats_elems(B, T, H), device="cuda"), B, T, H,
+                    p, seed, 1, ordered=True)
+        results.append(dqkv)
+    assert torch.equal(results[0], results[1]) and torch.equal(results[1], results[2])
+
+
+def test_long_contexts_keep_one_copy():
+    from zero_to_hero_b200.ops import native as N
+
+    assert N.flash_bwd_copies(16, 1024, 12) == 8 and N.flash_bwd_copies(1, 65536, 16) == 1

@@ -295,7 +295,8 @@ class GPT2TrainEngine:
             self.d_drop = buf(M, C)    # gradient of that output
         self.d_4c = buf(M, 4 * C)
         self.d_qkv = buf(M, 3 * C)
-        self.dq_accum = buf(N.flash_bwd_dq_elems(B, T, H), dtype=f32)
+        self.dq_copies = N.flash_bwd_copies(B, T, H) if self.cfg.train.deterministic else 1
+        self.dq_accum = buf(N.flash_bwd_dq_elems(B, T, H) * self.dq_copies, dtype=f32)
         self.attn_stats = buf(N.flash_bwd_stats_elems(B, T, H), dtype=f32)
         self.ln_scratch = buf(N.layernorm_bwd_num_partials(M) * 3 * C, dtype=f32)
 
@@ -533,8 +534,8 @@ class GPT2TrainEngine:
             self._on_side(wg_attn_proj)
             G.gemm(dy, w(p + "attn.c_proj.weight"), self.d_c, b_mn=True)
             # the c_attn bias gradient (column sums of d_qkv) comes out of the attention kernels; in
-            # the reproducible mode the attention backward runs one KV tile per launch (dQ accumulates
-            # in a fixed order) and the bias gradient is a single-writer column sum
+            # the reproducible mode the attention backward adds up dQ in KV-tile order and the bias
+            # gradient is a single-writer column sum
             det = self.deterministic
             N.flash_bwd(self.qkv[l], self.att[l], self.d_c, self.lse[l], self.d_qkv, self.dq_accum,
                         self.attn_stats, B, T, H, pd, seed, 1 + 3 * l,
@@ -557,9 +558,10 @@ class GPT2TrainEngine:
             # dgrad GEMMs, column-sum launches (the projection biases ride in the LayerNorm backward
             # without dropout, the QKV bias in the attention kernels, the c_fc bias usually in its
             # GEMM), LN bwd (2 kernels each), flash bwd (3)
-            # (reproducible mode: the attention backward is one launch per KV tile, plus the QKV column sum)
+            # (reproducible mode without memory for copies of dQ: one attention launch per KV tile; plus the
+            # QKV column sum)
             self._n += 4 + (0 if fuse_db else 2) + (0 if fc_db_in_gemm else 1) + 2 * 2
-            self._n += (2 + (T + 127) // 128 + 1) if det else 3
+            self._n += (2 + (1 if self.dq_copies > 1 else (T + 127) // 128) + 1) if det else 3
             if reduce:
                 self._reduce_ready(l)
         self._join_side()

@@ -28,6 +28,8 @@ _sigs = {
     "z2h_colsum_bf16_ordered": [c_void_p, c_int, c_int, c_longlong, c_void_p, c_int, c_int, c_void_p, c_void_p],
     "z2h_flash_bwd_ex": [c_void_p] * 7 + [c_int, c_int, c_int, c_float, c_void_p, ctypes.c_uint,
                          c_void_p, c_int, c_void_p, c_void_p],
+    "z2h_flash_bwd_sliced": [c_void_p] * 7 + [c_int, c_int, c_int, c_float, c_void_p, ctypes.c_uint,
+                             c_void_p, c_int, c_int, c_void_p, c_void_p],
     "z2h_ce_fwd_bwd": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_longlong,
                        c_float, c_int, c_int, c_void_p],
     "z2h_reduce_sum": [c_void_p, c_int, c_float, c_void_p, c_int, c_void_p],
@@ -182,22 +184,34 @@ def flash_bwd_dq_elems(B: int, T: int, H: int) -> int:
     return (B * T + 31) // 32 * 32 * H * 64
 
 
+ORDERED_DQ_BYTES = 512 << 20  # memory the copies of dQ may take
+
+
+def flash_bwd_copies(B: int, T: int, H: int) -> int:
+    """dq_accum copies worth having for the ordered form: one per 128-key tile, or 1 where they would take
+    more than ORDERED_DQ_BYTES (long contexts: their number and their size both grow with T)."""
+    n = (T + 127) // 128
+    return n if n * flash_bwd_dq_elems(B, T, H) * 4 <= ORDERED_DQ_BYTES else 1
+
+
 def flash_bwd(qkv, out, dout, lse, dqkv, dq_accum, stats, B, T, H, drop_p: float = 0.0, seed=None,
               site: int = 0, dbias=None, ordered: bool = False):
     """`dbias` (fp32 [3*H*64]): the column sums of `dqkv` as stored are ADDED to it, i.e. the gradient
     of the QKV projection's bias comes out of the attention backward kernels.
-    `ordered`: the KV tiles are launched one after the other, so the fp32 accumulation of dQ happens in
-    a fixed order (bitwise reproducible, about 1.5x slower; not together with `dbias`)."""
+    `ordered`: the fp32 accumulation of dQ happens in KV-tile order (bitwise reproducible; not together with
+    `dbias`). With `flash_bwd_copies` times the dq_accum scratch every KV tile stores to a copy of its own;
+    with less the KV tiles are launched one after the other (about 1.5x slower, the same bits)."""
     assert stats.numel() >= flash_bwd_stats_elems(B, T, H)
     assert dq_accum.numel() >= flash_bwd_dq_elems(B, T, H) and dq_accum.dtype == torch.float32
     if ordered:
         assert dbias is None, "the bias by-product is accumulated with atomics"
         if drop_p > 0.0:
             assert seed is not None and seed.dtype == torch.int64 and seed.is_cuda
-        _check(_f("z2h_flash_bwd_ex")(ptr(qkv), ptr(out), ptr(dout), ptr(lse), ptr(dqkv), ptr(dq_accum),
-                                      ptr(stats), B, T, H, drop_p, ptr(seed) if drop_p > 0.0 else None, site,
-                                      None, 1, ptr(_lib.status_word(out.device)), stream_ptr()),
-               "flash_bwd_ex")
+        _check(_f("z2h_flash_bwd_sliced")(ptr(qkv), ptr(out), ptr(dout), ptr(lse), ptr(dqkv), ptr(dq_accum),
+                                          ptr(stats), B, T, H, drop_p, ptr(seed) if drop_p > 0.0 else None, site,
+                                          None, 1, dq_accum.numel() // flash_bwd_dq_elems(B, T, H),
+                                          ptr(_lib.status_word(out.device)), stream_ptr()),
+               "flash_bwd_sliced")
         return
     if dbias is not None:
         assert dbias.dtype == torch.float32 and dbias.numel() == 3 * H * 64 and dbias.is_contiguous()
