@@ -58,8 +58,13 @@ int gemm_bf16(const GemmArgs& args, cudaStream_t stream);
 // The CTA-pair kernel (256 x 256 tiles, tcgen05.mma.cta_group::2); arguments already validated.
 int gemm_bf16_pair(const GemmArgs& args, cudaStream_t stream);
 
+// The one-CTA kernel with 128x64 and 128x128 tiles; arguments already validated.
+int gemm_bf16_narrow64(const GemmArgs& args, cudaStream_t stream);
+int gemm_bf16_narrow128(const GemmArgs& args, cudaStream_t stream);
+
 // 0: always the one-CTA kernel (128 x 256 tiles); 1: the CTA-pair kernel whenever M >= 256;
-// 2 (default): CTA pairs when the problem has at least one 256 x 256 tile per pair of SMs.
+// 2 (default): CTA pairs when the problem has at least one 256 x 256 tile per pair of SMs, else the
+// one-CTA kernel with the tile width pick_bn chooses; 64 or 128: always the one-CTA kernel of that width.
 void gemm_set_algo(int algo);
 // dst[i] += slices[0][i] + slices[1][i] + ... (in that order), n elements per slice, n % 4 == 0.
 int gemm_fold_slices(const float* slices, int num_slices, long long n, float* dst, cudaStream_t stream);

@@ -472,7 +472,7 @@ __device__ __forceinline__ void epilogue_block(const KernelParams& p, const uint
   }
 }
 
-// The warp's four blocks, two register buffers: while block c is worked on, the tensor-memory load
+// The warp's NB blocks (four in the 256-column tiles), two register buffers: while block c is worked on, the tensor-memory load
 // of block c + 1 and the load of its second operand (residual or pre-activation) are in flight. A
 // tensor-memory load issued while MMAs are queued takes around a thousand cycles and one row per
 // lane makes every global load a long-latency access of its own; with all four blocks loaded up
@@ -482,7 +482,7 @@ __device__ __forceinline__ void epilogue_block(const KernelParams& p, const uint
 //   taddr: tensor-memory address of the warp's first block; active: false for a tile that has no
 //   k-blocks in this worker's share (the accumulator protocol still runs).
 //   k_slice: which K-slice of the tile this is (kEpiSliceStore only; 0 otherwise)
-template <int EPI, bool OUT_FP32, class Release>
+template <int EPI, bool OUT_FP32, int NB, class Release>
 __device__ __forceinline__ void epilogue_stream(const KernelParams& p_in, uint32_t taddr, long long grow,
                                                 int gcol0, const float* sbias, int lane, uint32_t stage,
                                                 bool active, int k_slice, Release release) {
@@ -496,7 +496,7 @@ __device__ __forceinline__ void epilogue_stream(const KernelParams& p_in, uint32
   if (EPI == kEpiSliceStore) active = true;
   const bool row_ok = active && grow < p.M;
   const bool atomic_interior = OUT_FP32 && EPI == kEpiAtomicAdd && active && sbias == nullptr &&
-                               (grow - lane) + 32 <= p.M && gcol0 + 128 <= p.N;
+                               (grow - lane) + 32 <= p.M && gcol0 + NB * 32 <= p.N;
   const __nv_bfloat16* src = nullptr;
   if (EPI == kEpiResidual) src = p.residual + grow * p.ldr + gcol0;
   if (EPI == kEpiGeluGrad || EPI == kEpiMulAux) src = p.aux_in + grow * p.ldaux + gcol0;
@@ -506,7 +506,7 @@ __device__ __forceinline__ void epilogue_stream(const KernelParams& p_in, uint32
   tmem_ld_32x32b_x32(taddr, r[0]);
   if (kSecondOperand && row_ok && gcol0 + 32 <= p.N) ld_row(src, pre[0], wide);
 #pragma unroll 1
-  for (int c = 0; c < 4; c += 2) {
+  for (int c = 0; c < NB; c += 2) {
     tmem_ld_wait_for(r[0]);
     if (zero_fill) {
 #pragma unroll
@@ -521,7 +521,7 @@ __device__ __forceinline__ void epilogue_stream(const KernelParams& p_in, uint32
 #pragma unroll
       for (int j = 0; j < 32; ++j) r[1][j] = 0u;
     }
-    if (c + 2 < 4) {
+    if (c + 2 < NB) {
       tmem_ld_32x32b_x32(taddr + (c + 2) * 32, r[0]);
       if (kSecondOperand && row_ok && gcol0 + (c + 3) * 32 <= p.N) ld_row(src + (c + 2) * 32, pre[0], wide);
     } else {
@@ -541,35 +541,36 @@ __device__ __forceinline__ void epilogue_stream(const KernelParams& p_in, uint32
 // same kernel as the others they changed nothing in the other kinds' code, yet the register allocation
 // and scheduling of the whole kernel came out 10 % slower for every plain GEMM (M16384 N3072 K768
 // 63.5 -> 71.7 us, lm_head 932 -> 1020 us).
-template <bool EXTRA, class Release>
+// NB: 32-column blocks a warp drains (even; 4 for the 256-column tiles)
+template <bool EXTRA, int NB = 4, class Release>
 __device__ __forceinline__ void epilogue_tile_streamed(const KernelParams& p, uint32_t taddr, long long grow,
                                                        int gcol0, const float* sbias, int lane, uint32_t stage,
                                                        bool active, int k_slice, Release release) {
   if (EXTRA) {
     if (p.out_fp32)
-      return epilogue_stream<kEpiSliceStore, true>(p, taddr, grow, gcol0, sbias, lane, stage, active, k_slice, release);
+      return epilogue_stream<kEpiSliceStore, true, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, k_slice, release);
     if (p.epi == kEpiGeluSaveGrad)
-      return epilogue_stream<kEpiGeluSaveGrad, false>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
-    return epilogue_stream<kEpiMulAux, false>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+      return epilogue_stream<kEpiGeluSaveGrad, false, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+    return epilogue_stream<kEpiMulAux, false, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
   }
   if (p.out_fp32) {
     if (p.epi == kEpiAtomicAdd)
-      return epilogue_stream<kEpiAtomicAdd, true>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+      return epilogue_stream<kEpiAtomicAdd, true, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
     if (p.epi == kEpiAccumulate)
-      return epilogue_stream<kEpiAccumulate, true>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+      return epilogue_stream<kEpiAccumulate, true, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
     if (p.epi == kEpiNone)
-      return epilogue_stream<kEpiNone, true>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+      return epilogue_stream<kEpiNone, true, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
   } else {
     if (p.epi == kEpiNone)
-      return epilogue_stream<kEpiNone, false>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+      return epilogue_stream<kEpiNone, false, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
     if (p.epi == kEpiResidual)
-      return epilogue_stream<kEpiResidual, false>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+      return epilogue_stream<kEpiResidual, false, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
     if (p.epi == kEpiGelu)
-      return epilogue_stream<kEpiGelu, false>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+      return epilogue_stream<kEpiGelu, false, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
     if (p.epi == kEpiGeluGrad)
-      return epilogue_stream<kEpiGeluGrad, false>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+      return epilogue_stream<kEpiGeluGrad, false, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
   }
-  return epilogue_stream<kEpiGeneric, false>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
+  return epilogue_stream<kEpiGeneric, false, NB>(p, taddr, grow, gcol0, sbias, lane, stage, active, 0, release);
 }
 
 // Called before the wait for the accumulator: asks L2 for this lane's 128 columns (256 bytes) of the

@@ -90,7 +90,7 @@ def fold_slices(slices: torch.Tensor, num_slices: int, dst: torch.Tensor) -> Non
 
 def set_algo(algo: int) -> None:
     """0: one-CTA kernel (128x256 tiles); 1: CTA-pair kernel (256x256 tiles, cta_group::2) whenever
-    M >= 256; 2: automatic choice (default)."""
+    M >= 256; 2: automatic choice (default); 64 or 128: one-CTA kernel with tiles of that width."""
     _lib.cuda_lib().z2h_gemm_set_algo(int(algo))
 
 

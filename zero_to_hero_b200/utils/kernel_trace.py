@@ -27,7 +27,7 @@ from .. import build as _build
 
 TRACE_DIR = _build.ROOT / "build" / "trace"
 SOURCES = {
-    "gemm": ["gemm/gemm_tcgen05.cu", "gemm/gemm_tcgen05_2cta.cu", "common/tma_desc.cu"],
+    "gemm": ["gemm/gemm_tcgen05.cu", "gemm/gemm_narrow64.cu", "gemm/gemm_narrow128.cu", "gemm/gemm_tcgen05_2cta.cu", "common/tma_desc.cu"],
     "flash_bwd": ["attn/flash_bwd.cu", "common/tma_desc.cu"],
     "flash_fwd": ["attn/flash_fwd.cu", "common/tma_desc.cu"],
 }
