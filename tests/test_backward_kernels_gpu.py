@@ -70,3 +70,21 @@ def test_long_contexts_keep_one_copy():
     from zero_to_hero_b200.ops import native as N
 
     assert N.flash_bwd_copies(16, 1024, 12) == 8 and N.flash_bwd_copies(1, 65536, 16) == 1
+
+
+# fewer positions than vocabulary rows (a warp per position) and as many (a warp per row); more than one
+# chunk of ids and of columns; tokens that occur often, once, never and out of range
+@pytest.mark.parametrize("B,T,C,V", [(1, 1, 8, 2), (3, 70, 264, 1000), (5, 509, 384, 50257), (2, 3000, 264, 6000)])
+def test_ordered_embedding_gradient(B, T, C, V):
+    from zero_to_hero_b200.ops import native as N
+
+    g = torch.Generator().manual_seed(T)
+    idx = torch.randint(0, V, (B, T), generator=g)
+    idx[:, ::3] = idx[0, 0]
+    idx[-1, -1] = V + 5  # clamped into the table
+    dx = torch.randn(B * T, C, generator=g).bfloat16()
+    want = torch.zeros(V, C).index_add_(0, idx.clamp(0, V - 1).flatten(), dx.float())  # ascending, fp32
+    for dtype in (torch.int64, torch.int32):
+        dwte, dwpe = torch.zeros(V, C, device="cuda"), torch.zeros(T, C, device="cuda")
+        N.embed_bwd(idx.to(dtype).cuda(), dx.cuda(), dwte, dwpe, B, T, ordered=True)
+        assert torch.equal(dwte.cpu(), want)
