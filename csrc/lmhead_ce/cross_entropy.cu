@@ -254,6 +254,140 @@ ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const IdxT* __restrict__ t
   }
 }
 
+// ---- out of place, for autograd: the forward keeps a copy of the logits, the backward is one pass over it
+// The forward reads a row once and writes its copy (the caller may go on to change its logits); one bulk
+// copy in, two passes over shared memory (maximum, sum of exponentials), one bulk copy out. Rows that do
+// not start on 16 bytes (an odd vocabulary, SHIFT) are read from the boundary below and written aligned
+// from registers, so that everything that follows works on an aligned pitch.
+struct RowWindow {
+  const uint32_t* words;  // shared memory
+  int shift;              // columns between the copy's start and the row's
+  // columns 8v .. 8v+7 of the row as packed pairs
+  template <bool SHIFT>
+  __device__ __forceinline__ uint4 vec(int v) const {
+    if (!SHIFT) return reinterpret_cast<const uint4*>(words)[v];
+    const int at = shift + 8 * v;
+    const uint32_t* w = words + (at >> 1);
+    if ((at & 1) == 0) return make_uint4(w[0], w[1], w[2], w[3]);
+    const uint32_t a = w[0], b = w[1], c = w[2], d = w[3], e = w[4];
+    return make_uint4(__funnelshift_r(a, b, 16), __funnelshift_r(b, c, 16), __funnelshift_r(c, d, 16),
+                      __funnelshift_r(d, e, 16));
+  }
+};
+
+template <typename IdxT, bool SHIFT>
+__global__ void __launch_bounds__(kRowThreads)
+ce_fwd_save_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, const IdxT* __restrict__ targets,
+                   float* __restrict__ losses, float* __restrict__ lse_out, __nv_bfloat16* __restrict__ copy,
+                   long long ld_copy, int V, int V_real, int ignore_index, int* status) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ float sh[32];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ int abort_flag;
+  const int row = blockIdx.x, nvec = (V + 7) / 8;
+  const __nv_bfloat16* lr = logits + (long long)row * ld;
+  RowWindow win;
+  win.words = reinterpret_cast<const uint32_t*>(smem);
+  win.shift = SHIFT ? (int)((reinterpret_cast<uintptr_t>(lr) & 15) / 2) : 0;
+  const uint32_t bytes = (uint32_t)(((win.shift + V) * 2 + 15) / 16 * 16);
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    abort_flag = 0;
+    fence_mbar_init();
+    mbar_arrive_expect_tx(&bar, bytes);
+    bulk_load_1d(smem, lr - win.shift, bytes, &bar);
+  }
+  __syncthreads();
+  const long long tgt = (long long)targets[row];
+  const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V_real;
+  if (!mbar_wait_bounded(&bar, 0, &abort_flag, status, kTimeoutFull)) return;
+  if (!SHIFT && copy != nullptr && threadIdx.x == 0) {
+    bulk_store_1d(copy + (long long)row * ld_copy, smem, bytes);
+    tma_store_commit();
+  }
+  float m = -INFINITY;
+  for (int v = threadIdx.x; v < nvec; v += kRowThreads) {
+    uint4 u = win.vec<SHIFT>(v);
+    uint32_t* w = &u.x;
+    if (SHIFT && v * 8 + 8 > V) {  // past the row's end lies the next row: zeros in the copy
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (v * 8 + 2 * j >= V) w[j] = 0;
+        else if (v * 8 + 2 * j + 1 >= V) w[j] &= 0xffffu;
+      }
+    }
+    if (SHIFT && copy != nullptr) *reinterpret_cast<uint4*>(copy + (long long)row * ld_copy + v * 8) = u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = unpack_bf16x2(w[j]);
+      const int c = v * 8 + 2 * j;
+      if (c < V_real) m = fmaxf(m, f.x);
+      if (c + 1 < V_real) m = fmaxf(m, f.y);
+    }
+  }
+  m = cta_reduce<true>(m, sh);
+  const float m2 = m * kLog2e;
+  float s = 0.f;
+  for (int v = threadIdx.x; v < nvec; v += kRowThreads) {
+    const uint4 u = win.vec<SHIFT>(v);
+    const uint32_t* w = &u.x;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = unpack_bf16x2(w[j]);
+      const int c = v * 8 + 2 * j;
+      const float e0 = ex2_fast(fmaf(f.x, kLog2e, -m2)), e1 = ex2_fast(fmaf(f.y, kLog2e, -m2));
+      s += (c < V_real ? e0 : 0.f) + (c + 1 < V_real ? e1 : 0.f);
+    }
+  }
+  s = cta_reduce<false>(s, sh);
+  if (threadIdx.x == 0) {
+    const float lse = m + logf(s);
+    lse_out[row] = lse;
+    losses[row] = ignored ? 0.f : lse - __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(smem)[win.shift + tgt]);
+    if (!SHIFT && copy != nullptr) tma_store_wait_read<0>();  // shared memory stays until the copy has read it
+  }
+}
+
+// grad = (exp(x - lse) - onehot) * scale * *upstream: one read, one write, rounded once. Two rows in
+// flight per SM hide the loads; a thread keeps four vectors in flight.
+template <typename IdxT>
+__global__ void __launch_bounds__(kThreads)
+ce_bwd_kernel(const __nv_bfloat16* __restrict__ x, const IdxT* __restrict__ targets, const float* __restrict__ lse,
+              const float* __restrict__ upstream, float scale, __nv_bfloat16* __restrict__ grad, long long ld, int V,
+              int V_real, int ignore_index) {
+  const int row = blockIdx.x, nvec = (V + 7) / 8;
+  const long long tgt = (long long)targets[row];
+  const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V_real;
+  const float g = ignored ? 0.f : *upstream * scale, l2 = lse[row] * kLog2e;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + (long long)row * ld);
+  uint4* gr = reinterpret_cast<uint4*>(grad + (long long)row * ld);
+#pragma unroll 4
+  for (int v = threadIdx.x; v < nvec; v += kThreads) {
+    uint4 u = xr[v];
+    uint32_t* w = &u.x;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = unpack_bf16x2(w[j]);
+      const int c = v * 8 + 2 * j;
+      float a = ex2_fast(fmaf(f.x, kLog2e, -l2)), b = ex2_fast(fmaf(f.y, kLog2e, -l2));
+      if (c == tgt) a -= 1.f;
+      if (c + 1 == tgt) b -= 1.f;
+      w[j] = pack_bf16x2(c < V_real && !ignored ? a * g : 0.f, c + 1 < V_real && !ignored ? b * g : 0.f);
+    }
+    gr[v] = u;
+  }
+}
+
+// dst[m][c] (tight rows of any width) = src[m][c] (rows on an aligned pitch). Two bytes a lane, eight in
+// flight: the rows of an odd width share no alignment with their source.
+__global__ void __launch_bounds__(256)
+compact_rows_kernel(const __nv_bfloat16* __restrict__ src, long long ld, __nv_bfloat16* __restrict__ dst, int N) {
+  const long long row = blockIdx.x;
+#pragma unroll 8
+  for (int c = threadIdx.x + blockIdx.y * 8192; c < min(N, (int)(blockIdx.y + 1) * 8192); c += 256)
+    dst[row * N + c] = src[row * ld + c];
+}
+
 // Sum of n floats into *out (scaled); single CTA, fixed order.
 __global__ void reduce_sum_kernel(const float* __restrict__ x, int n, float scale, float* out,
                                   int accumulate) {
@@ -313,6 +447,54 @@ int ce_fwd_bwd(void* logits, const void* targets, int idx_is_64, float* losses, 
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
+template <typename IdxT>
+static int ce_fwd_save_t(const void* logits, long long ld, const void* targets, float* losses, float* lse, void* copy,
+                         long long ld_copy, int M, int V, int V_real, int ignore_index, cudaStream_t stream) {
+  const bool shift = (ld % 8) != 0 || (reinterpret_cast<uintptr_t>(logits) & 15) || V % 8 != 0;
+  const size_t smem = (size_t)((V + 7 + 7) / 8 * 8 + 8) * 2;  // the row, up to 7 columns before it, a word after
+  if (smem > (size_t)kRowMaxBytes) return 1;
+  static std::atomic<unsigned long long> seen{0};
+  if (first_use_on_current_device(seen)) {
+    cudaFuncSetAttribute(ce_fwd_save_kernel<IdxT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowMaxBytes);
+    cudaFuncSetAttribute(ce_fwd_save_kernel<IdxT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowMaxBytes);
+  }
+  auto kern = shift ? ce_fwd_save_kernel<IdxT, true> : ce_fwd_save_kernel<IdxT, false>;
+  kern<<<M, kRowThreads, smem, stream>>>((const __nv_bfloat16*)logits, ld, (const IdxT*)targets, losses, lse,
+                                         (__nv_bfloat16*)copy, ld_copy, V, V_real, ignore_index, nullptr);
+  return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
+
+int ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* lse,
+                void* copy, long long ld_copy, int M, int V, int V_real, int ignore_index, cudaStream_t stream) {
+  if (M <= 0) return 0;
+  if (V < 1 || V_real < 1 || V_real > V || ld < V || (reinterpret_cast<uintptr_t>(logits) & 1)) return 1;
+  if (copy != nullptr && (ld_copy % 8 || ld_copy < (V + 7) / 8 * 8 || (reinterpret_cast<uintptr_t>(copy) & 15))) return 1;
+  return idx_is_64 ? ce_fwd_save_t<long long>(logits, ld, targets, losses, lse, copy, ld_copy, M, V, V_real, ignore_index, stream)
+                   : ce_fwd_save_t<int>(logits, ld, targets, losses, lse, copy, ld_copy, M, V, V_real, ignore_index, stream);
+}
+
+int ce_bwd(const void* x, const void* targets, int idx_is_64, const float* lse, const float* upstream, float scale,
+           void* grad, long long ld, int M, int V, int V_real, int ignore_index, cudaStream_t stream) {
+  if (M <= 0) return 0;
+  if (V < 1 || V_real < 1 || V_real > V || ld % 8 || ld < (V + 7) / 8 * 8 ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(grad)) & 15))
+    return 1;
+  if (idx_is_64)
+    ce_bwd_kernel<long long><<<M, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (const long long*)targets, lse, upstream,
+                                                         scale, (__nv_bfloat16*)grad, ld, V, V_real, ignore_index);
+  else
+    ce_bwd_kernel<int><<<M, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (const int*)targets, lse, upstream, scale,
+                                                   (__nv_bfloat16*)grad, ld, V, V_real, ignore_index);
+  return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
+
+int compact_rows(const void* src, long long ld, void* dst, int M, int N, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (ld < N) return 1;
+  compact_rows_kernel<<<dim3(M, (N + 8191) / 8192), 256, 0, stream>>>((const __nv_bfloat16*)src, ld, (__nv_bfloat16*)dst, N);
+  return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
+
 int reduce_sum(const float* x, int n, float scale, float* out, int accumulate, cudaStream_t stream) {
   launch_kernel(reduce_sum_kernel, dim3(1), dim3(1024), 0, stream, true, x, n, scale, out, accumulate);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
@@ -326,6 +508,19 @@ int z2h_ce_fwd_bwd(void* logits, const void* targets, int idx_is_64, float* loss
                    void* stream) {
   return z2h::ce_fwd_bwd(logits, targets, idx_is_64, losses, M, V_real, V_pad, ld, grad_scale,
                          write_grad, ignore_index, (cudaStream_t)stream);
+}
+int z2h_ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* lse,
+                    void* copy, long long ld_copy, int M, int V, int V_real, int ignore_index, void* stream) {
+  return z2h::ce_fwd_save(logits, ld, targets, idx_is_64, losses, lse, copy, ld_copy, M, V, V_real, ignore_index,
+                          (cudaStream_t)stream);
+}
+int z2h_ce_bwd(const void* x, const void* targets, int idx_is_64, const float* lse, const float* upstream, float scale,
+               void* grad, long long ld, int M, int V, int V_real, int ignore_index, void* stream) {
+  return z2h::ce_bwd(x, targets, idx_is_64, lse, upstream, scale, grad, ld, M, V, V_real, ignore_index,
+                     (cudaStream_t)stream);
+}
+int z2h_compact_rows(const void* src, long long ld, void* dst, int M, int N, void* stream) {
+  return z2h::compact_rows(src, ld, dst, M, N, (cudaStream_t)stream);
 }
 int z2h_reduce_sum(const float* x, int n, float scale, float* out, int accumulate, void* stream) {
   return z2h::reduce_sum(x, n, scale, out, accumulate, (cudaStream_t)stream);

@@ -1,0 +1,105 @@
+"""Autograd ops against fp64 PyTorch: cross-entropy of any vocabulary, linear layers of any output width
+and the GELU backward."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+BF16 = 2.0 ** -8  # a rounding to bf16 is off by at most 2^-9; two meet where a second one follows
+
+
+def _rel(a, b):
+    a, b = a.double().cpu(), b.double().cpu()
+    return float((a - b).norm() / b.norm().clamp_min(1e-30))
+
+
+# one row, rows of one vector, an odd start of every row, the usual vocabularies, the widest row that fits
+@pytest.mark.parametrize("M,V", [(1, 8), (3, 65), (5, 1001), (129, 50257), (64, 50304), (7, 57297), (2, 57296)])
+def test_cross_entropy(M, V):
+    from zero_to_hero_b200.ops import functional as Z
+
+    g = torch.Generator().manual_seed(M + V)
+    x = (4 * torch.randn(M, V, generator=g)).bfloat16().cuda().requires_grad_()
+    t = torch.randint(0, V, (M,), generator=g).cuda()
+    if M > 2:
+        t[1] = -100
+    ref = x.detach().double().requires_grad_()
+    losses = F.cross_entropy(ref, t, reduction="none")  # zero for an ignored row
+    (losses.sum() / ((t != -100).sum() if V % 8 else M) * 3.0).backward()
+    logits = x * 1.0
+    loss = Z.cross_entropy(logits, t)
+    with torch.no_grad():
+        logits.zero_()  # the caller's logits are free once the loss is there
+    (loss * 3.0).backward(retain_graph=True)
+    first, x.grad = x.grad, None
+    (loss * 3.0).backward()
+    assert torch.equal(first, x.grad)
+    value = float(loss.detach())
+    assert abs(value - float(losses.detach().sum() / ((t != -100).sum() if V % 8 else M))) < 1e-4 * value
+    assert _rel(x.grad, ref.grad) < BF16
+    if M > 2:
+        assert not x.grad[1].any()
+    with torch.no_grad():
+        assert torch.equal(Z.cross_entropy(x * 1.0, t), loss)
+
+
+def test_cross_entropy_other_forms_keep_their_results():
+    from zero_to_hero_b200.ops import functional as Z
+
+    g = torch.Generator().manual_seed(0)
+    x = torch.randn(6, 40, generator=g).bfloat16().cuda()
+    t = torch.randint(0, 33, (6,), generator=g).cuda()
+    ref = F.cross_entropy(x[:, :33].double(), t)
+    for form in (x, x.float(), torch.cat((x, x), 1)[:, :40], torch.stack((x, x), 2)[:, :, 0]):
+        assert abs(float(Z.cross_entropy(form, t, 33)) - float(ref)) < 1e-4
+        assert abs(float(Z.cross_entropy(form, t.int(), 33)) - float(ref)) < 1e-4
+    y = x[:, :33].contiguous().requires_grad_()  # an odd vocabulary can be differentiated twice
+    d = y.detach().double().requires_grad_()
+    for v in (y, d):
+        loss = Z.cross_entropy(v, t) if v is y else F.cross_entropy(v, t)
+        (grad,) = torch.autograd.grad(loss, v, create_graph=True)
+        grad.square().sum().backward()
+    assert _rel(y.grad, d.grad) < 4 * BF16
+    lowest = torch.full((2, 33), torch.finfo(torch.bfloat16).min, dtype=torch.bfloat16, device="cuda")
+    lowest[:, 5] = 1.0
+    lowest[:, 6] = -torch.inf
+    assert float(Z.cross_entropy(lowest, torch.tensor([5, 5], device="cuda"))) == 0.0
+
+
+@pytest.mark.parametrize("M,K,N,bias", [(1, 8, 1, True), (300, 384, 65, True), (130, 64, 127, False),
+                                        (2048, 64, 257, True), (33, 768, 50257, False)])
+def test_linear_of_any_width(M, K, N, bias):
+    from zero_to_hero_b200.ops import functional as Z
+
+    Z.FALLBACK_COUNTS.clear()
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, K, generator=g).cuda().requires_grad_()
+    w = (torch.randn(N, K, generator=g) / K ** 0.5).cuda().requires_grad_()
+    b = torch.randn(N, generator=g).cuda().requires_grad_() if bias else None
+    dy = torch.randn(M, N, generator=g).cuda()
+    y = Z.linear(x, w, b)
+    y.backward(dy.bfloat16())
+    assert not Z.FALLBACK_COUNTS and y.is_contiguous() and y.dtype == torch.bfloat16
+    rx, rw = x.detach().bfloat16().double().requires_grad_(), w.detach().bfloat16().double().requires_grad_()
+    rb = b.detach().bfloat16().double().requires_grad_() if bias else None
+    r = F.linear(rx, rw, rb)
+    r.backward(dy.bfloat16().double())
+    assert _rel(y, r) < BF16 and _rel(x.grad, rx.grad) < BF16 and _rel(w.grad, rw.grad) < BF16
+    assert not bias or _rel(b.grad, rb.grad) < BF16
+
+
+@pytest.mark.parametrize("M,N", [(1, 8), (33, 264), (1000, 256), (4099, 3072)])
+def test_gelu_backward(M, N):
+    from zero_to_hero_b200.ops import native
+
+    g = torch.Generator().manual_seed(M)
+    pre = (3 * torch.randn(M, N, generator=g)).bfloat16().cuda()
+    pre[0, :4] = torch.tensor([0.0, 40.0, -40.0, 1e30])
+    dy = torch.randn(M, N, generator=g).bfloat16().cuda()
+    ref = pre.double().requires_grad_()
+    F.gelu(ref, approximate="tanh").backward(dy.double())
+    dx, db = torch.empty_like(dy), torch.ones(N, device="cuda")
+    native.gelu_bwd(dy, pre, dx, db)
+    ok = torch.isfinite(ref.grad)  # fp64's own x^3 stays finite where fp32's overflows: both end at 0 or dy
+    assert _rel(dx[ok], ref.grad[ok]) < BF16 and torch.isfinite(dx).all()
+    assert torch.allclose(db.double(), 1 + dx.double().sum(0), rtol=1e-4, atol=1e-4 * M ** 0.5)

@@ -6,7 +6,7 @@ back to plain PyTorch in the input dtype, which is also the fp32 oracle the kern
 compare against. There is no silent fallback on a GPU: if the native library is missing the
 call raises.
 
-Shapes the tensor-core GEMM cannot take (inner sizes that are not multiples of 8 elements,
+Shapes the tensor-core GEMM cannot take (contracted sizes that are not multiples of 8 elements,
 i.e. 16 bytes for TMA) are routed to `torch.matmul` in bf16 and counted in
 `FALLBACK_COUNTS` so tests can assert the hot shapes never take that route.
 """
@@ -114,9 +114,16 @@ class _Linear(torch.autograd.Function):
         dy2 = dy.reshape(M, Nout)
         dy2 = (dy2 if dy2.dtype == torch.bfloat16 else dy2.bfloat16()).contiguous()
         dres = dy2.reshape(dy.shape).to(ctx.res_dtype) if ctx.has_res else None
-        if pre is not None:
-            dy2 = _gelu_grad_mul(dy2, pre)  # dpre = dy * gelu'(pre)
-        dx = dw = db = None
+        dx = dw = db32 = None
+        want_db = ctx.has_bias and ctx.needs_input_grad[2]
+        if want_db:
+            db32 = torch.zeros(Nout, device=dy.device, dtype=torch.float32)
+        if pre is not None:  # dpre = dy * gelu'(pre), its column sums on the way
+            dpre = torch.empty_like(pre)
+            N.gelu_bwd(dy2, pre, dpre, db32)
+            dy2 = dpre
+        elif want_db:
+            N.colsum_bf16(dy2, db32, accumulate=True)
         if ctx.needs_input_grad[0]:
             dx2 = torch.empty(M, K, device=dy.device, dtype=torch.bfloat16)
             G.gemm(dy2, w16, dx2, b_mn=True)
@@ -127,20 +134,66 @@ class _Linear(torch.autograd.Function):
             sk = pick_split_k(tiles, math.ceil(M / 64))
             G.gemm(dy2, x2, dw32, a_mn=True, b_mn=True, epi=G.EPI_ATOMIC_ADD, split_k=sk)
             dw = dw32.to(ctx.w_dtype)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            db32 = torch.zeros(Nout, device=dy.device, dtype=torch.float32)
-            N.colsum_bf16(dy2, db32, accumulate=True)
-            db = db32.to(ctx.b_dtype)
-        return dx, dw, db, None, dres
+        return dx, dw, None if db32 is None else db32.to(ctx.b_dtype), None, dres
 
 
-def _gelu_grad_mul(dy: torch.Tensor, pre: torch.Tensor) -> torch.Tensor:
-    x = pre.float()
-    k0, k1 = 0.7978845608028654, 0.044715
-    u = k0 * (x + k1 * x * x * x)
-    t = torch.tanh(u)
-    g = 0.5 * (1 + t) + 0.5 * x * (1 - t * t) * k0 * (1 + 3 * k1 * x * x)
-    return (dy.float() * g).bfloat16()
+def _transformed() -> bool:
+    """Inside a function transform (vmap, torch.func.grad) or forward-mode differentiation."""
+    return torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0
+
+
+def _tight(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and on the 16-byte boundary the tensor maps need."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+class _LinearAnyWidth(torch.autograd.Function):
+    """y = x @ w.T + b over bf16 tensors for output widths that are no multiple of 8 (an unpadded
+    vocabulary): the tensor cores work on a 16-byte pitch, the caller gets tight rows."""
+
+    @staticmethod
+    def forward(ctx, x, w, b):
+        Nout, K = w.shape
+        x2 = _tight(x.reshape(-1, K))
+        M = x2.shape[0]
+        wide = torch.empty(M, (Nout + 7) // 8 * 8, device=x.device, dtype=torch.bfloat16)
+        G.gemm(x2, _tight(w), wide[:, :Nout], bias=None if b is None else _tight(b))
+        y = torch.empty(M, Nout, device=x.device, dtype=torch.bfloat16)
+        N.compact_rows(wide, y)
+        ctx.save_for_backward(x, w)
+        ctx.has_bias = b is not None
+        return y.reshape(*x.shape[:-1], Nout)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, w = ctx.saved_tensors
+        Nout, K = w.shape
+        need_x, need_w, need_b = ctx.needs_input_grad
+        d2, x2 = dy.reshape(-1, Nout), x.reshape(-1, K)
+        if torch.is_grad_enabled():  # a graph of this backward is wanted: plain operations
+            return ((d2 @ w).reshape(x.shape) if need_x else None, d2.t() @ x2 if need_w else None,
+                    d2.sum(0) if need_b else None)
+        M = d2.shape[0]
+        if d2.stride(1) != 1 or d2.stride(0) % 8 or d2.stride(0) < Nout or d2.data_ptr() % 16:
+            d2 = d2.new_empty(M, (Nout + 7) // 8 * 8)[:, :Nout].copy_(d2)
+        dx = dw = db = None
+        if need_x:
+            dx = torch.empty(M, K, device=dy.device, dtype=torch.bfloat16)
+            G.gemm(d2, _tight(w), dx, b_mn=True)
+            dx = dx.reshape(x.shape)
+        if need_w:
+            sk = pick_split_k(math.ceil(Nout / 128) * math.ceil(K / 256), math.ceil(M / 64))
+            if sk == 1:
+                dw = torch.empty(Nout, K, device=dy.device, dtype=torch.bfloat16)
+                G.gemm(d2, _tight(x2), dw, a_mn=True, b_mn=True)
+            else:
+                dw = torch.zeros(Nout, K, device=dy.device, dtype=torch.float32)
+                G.gemm(d2, _tight(x2), dw, a_mn=True, b_mn=True, epi=G.EPI_ATOMIC_ADD, split_k=sk)
+                dw = dw.bfloat16()
+        if need_b:
+            db = d2.sum(0, dtype=torch.float32).bfloat16()
+        return dx, dw, db
 
 
 def linear(x, w, b=None, act: str | None = None, residual=None):
@@ -149,6 +202,9 @@ def linear(x, w, b=None, act: str | None = None, residual=None):
     K, Nout = x.shape[-1], w.shape[0]
     if _native(x) and _gemm_ok(K, Nout):
         return _Linear.apply(x, w, b, act, residual)
+    if _native(x) and _gemm_ok(K) and act is None and residual is None and w.dim() == 2 and x.numel() > 0 and \
+            w.numel() > 0 and not _transformed():
+        return _LinearAnyWidth.apply(x.bfloat16(), w.bfloat16(), None if b is None else b.bfloat16())
     if _native(x):
         FALLBACK_COUNTS["linear"] += 1
         y = F.linear(x.bfloat16(), w.bfloat16(), None if b is None else b.bfloat16())
@@ -320,12 +376,62 @@ class _CrossEntropy(torch.autograd.Function):
         return (dlogits.float() * g).to(ctx.dtype), None, None
 
 
+class _CrossEntropySaved(torch.autograd.Function):
+    """The same over bf16 logits whose rows are tight in memory, any vocabulary: one pass forward that keeps
+    a copy of the logits (the caller's may change before the backward), one pass backward that rounds the
+    gradient once. `skip_ignored`: the mean is over the targets that are not ignored."""
+
+    @staticmethod
+    def forward(ctx, logits, targets, v_real, skip_ignored):
+        M, V = logits.shape
+        targets = targets.contiguous()
+        losses = torch.empty(M, device=logits.device, dtype=torch.float32)
+        lse = torch.empty_like(losses)
+        copy = None
+        if ctx.needs_input_grad[0]:
+            copy = torch.empty(M, (V + 7) // 8 * 8, device=logits.device, dtype=torch.bfloat16)
+        N.ce_fwd_save(logits, targets, losses, lse, copy, v_real)
+        count = (targets != -100).sum().float() if skip_ignored else None
+        if copy is not None:
+            ctx.save_for_backward(copy, targets, lse, count)
+            ctx.meta = (M, V, v_real)
+            # a second derivative goes through the caller's logits themselves
+            ctx.logits, ctx.version = (logits, logits._version) if skip_ignored else (None, 0)
+        return losses.mean() if count is None else losses.sum() / count
+
+    @staticmethod
+    def backward(ctx, g):
+        copy, targets, lse, count = ctx.saved_tensors
+        M, V, v_real = ctx.meta
+        skipping = count is not None
+        if torch.is_grad_enabled() and (g.requires_grad or skipping):  # a graph of this backward is wanted
+            x = ctx.logits if skipping and ctx.logits._version == ctx.version else copy
+            x = x[:, :v_real].float()
+            valid = ((targets >= 0) & (targets < v_real)).float()
+            hit = (targets[:, None] == torch.arange(v_real, device=x.device)).float()
+            p = x.softmax(1) if skipping else torch.exp(x - lse[:, None])
+            grad = F.pad((p - hit) * valid[:, None], (0, V - v_real))
+            return (grad * (g / count if skipping else g / M)).bfloat16(), None, None, None
+        grad = torch.empty_like(copy)
+        up = g / count if skipping else g
+        N.ce_bwd(copy, targets, lse, up.reshape(1), 1.0 if skipping else 1.0 / M, grad, V, v_real)
+        return grad[:, :V], None, None, None
+
+
 def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, v_real: int | None = None) -> torch.Tensor:
     """Mean softmax cross-entropy over rows; columns >= v_real are vocabulary padding."""
     V = logits.shape[-1]
     v_real = V if v_real is None else v_real
-    if _native(logits) and V % 8 == 0:
-        return _CrossEntropy.apply(logits.reshape(-1, V), targets.reshape(-1), v_real)
+    if _native(logits):
+        x, t = logits.reshape(-1, V), targets.reshape(-1)
+        tight = (x.dtype == torch.bfloat16 and V <= N.CE_SAVE_MAX_COLUMNS and 1 <= v_real <= V and x.shape[0] > 0
+                 and t.shape[0] == x.shape[0] and x.is_contiguous())
+        if V % 8 == 0:
+            if tight and t.dtype in (torch.int64, torch.int32):
+                return _CrossEntropySaved.apply(x, t, v_real, False)
+            return _CrossEntropy.apply(x, t, v_real)
+        if tight and t.dtype == torch.int64 and t.device == x.device and not _transformed():
+            return _CrossEntropySaved.apply(x, t, v_real, True)
     if _native(logits):
         FALLBACK_COUNTS["cross_entropy"] += 1
     return F.cross_entropy(logits.reshape(-1, V)[:, :v_real].float(), targets.reshape(-1))

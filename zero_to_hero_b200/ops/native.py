@@ -32,6 +32,12 @@ _sigs = {
                              c_void_p, c_int, c_int, c_void_p, c_void_p],
     "z2h_ce_fwd_bwd": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_longlong,
                        c_float, c_int, c_int, c_void_p],
+    "z2h_ce_fwd_save": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int,
+                        c_int, c_int, c_void_p],
+    "z2h_ce_bwd": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, c_longlong, c_int, c_int, c_int,
+                   c_int, c_void_p],
+    "z2h_compact_rows": [c_void_p, c_longlong, c_void_p, c_int, c_int, c_void_p],
+    "z2h_gelu_bwd": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "z2h_reduce_sum": [c_void_p, c_int, c_float, c_void_p, c_int, c_void_p],
     "z2h_gradnorm_partials": [c_void_p, c_longlong, c_void_p, c_void_p],
     "z2h_adamw_step": [c_void_p] * 5 + [c_longlong, c_longlong, c_void_p, c_void_p, c_int,
@@ -119,6 +125,38 @@ def ce_fwd_bwd(logits, targets, losses, v_real, grad_scale, write_grad=True, ign
     _check(_f("z2h_ce_fwd_bwd")(ptr(logits), ptr(targets), _is64(targets), ptr(losses), M, v_real,
                                 Vp, logits.stride(0), grad_scale, int(write_grad), ignore_index,
                                 stream_ptr()), "ce_fwd_bwd")
+
+
+CE_SAVE_MAX_COLUMNS = 57_300  # a row of logits lies in shared memory, two rows to an SM
+
+
+def ce_fwd_save(logits, targets, losses, lse, copy, v_real, ignore_index=-100):
+    """Losses and log-sum-exps of the rows of `logits` [M, V] (bf16, unit inner stride, any pitch); `copy`
+    ([M, >= V] on a pitch of a multiple of 8, or None) receives the logits for `ce_bwd`."""
+    M, V = logits.shape
+    _check(_f("z2h_ce_fwd_save")(ptr(logits), max(logits.stride(0), V) if M == 1 else logits.stride(0), ptr(targets),
+                                 _is64(targets), ptr(losses), ptr(lse), ptr(copy),
+                                 0 if copy is None else copy.stride(0), M, V, v_real, ignore_index, stream_ptr()),
+           "ce_fwd_save")
+
+
+def ce_bwd(copy, targets, lse, upstream, scale, grad, V, v_real, ignore_index=-100):
+    """grad = (softmax - onehot) * scale * upstream[0]; `copy` and `grad` share one pitch."""
+    assert copy.stride(0) == grad.stride(0) and upstream.dtype == torch.float32
+    _check(_f("z2h_ce_bwd")(ptr(copy), ptr(targets), _is64(targets), ptr(lse), ptr(upstream), scale, ptr(grad),
+                            copy.stride(0), copy.shape[0], V, v_real, ignore_index, stream_ptr()), "ce_bwd")
+
+
+def compact_rows(src, dst):
+    """Tight dst [M, N] = src [M, N] on a wider pitch (bf16)."""
+    _check(_f("z2h_compact_rows")(ptr(src), src.stride(0), ptr(dst), dst.shape[0], dst.shape[1], stream_ptr()),
+           "compact_rows")
+
+
+def gelu_bwd(dy, pre, dx, db=None):
+    """dx = dy * gelu_tanh'(pre) over tight bf16 [M, N]; `db` (fp32 [N]) += column sums of dx."""
+    M, N = pre.shape
+    _check(_f("z2h_gelu_bwd")(ptr(dy), ptr(pre), ptr(dx), ptr(db), M, N, stream_ptr()), "gelu_bwd")
 
 
 def reduce_sum(x, out, scale=1.0, accumulate=False):
