@@ -1,0 +1,155 @@
+"""Cached decoding: the rules that send a call there (CPU) and its results (GPU)."""
+import copy
+
+import pytest
+import torch
+import torch.nn as nn
+
+from zero_to_hero_b200.config import ModelConfig
+from zero_to_hero_b200.models.gpt2 import GPT2
+from zero_to_hero_b200.ops import decode
+
+
+def _model(heads=2, layers=2, vocab=101, block=40, ln_bias=False, dropout=0.0, seed=0):
+    torch.manual_seed(seed)
+    cfg = ModelConfig(vocab_size=vocab, block_size=block, emb_dim=64 * heads, num_heads=heads, num_layers=layers,
+                      dropout=dropout, ln_bias=ln_bias)
+    m = GPT2(cfg)
+    with torch.no_grad():  # biases and norm weights that matter, logits that spread
+        for n, p in m.named_parameters():
+            if p.dim() < 2:
+                p.add_(0.1 * torch.randn_like(p))
+        m.transformer.wte.weight.normal_(0.0, 0.3)
+        m.transformer.wpe.weight.normal_(0.0, 0.3)
+    return m.eval()
+
+
+@pytest.mark.parametrize("ln_bias", (False, True))
+def test_packed_layout_holds_every_parameter_once(ln_bias):
+    m = _model(heads=3, layers=3, vocab=77, ln_bias=ln_bias)
+    off, numbers, total = decode.packed_layout(m.config)
+    spans = sorted((off[n], off[n] + p.numel()) for n, p in m.named_parameters())
+    assert len(spans) == len(off) and all(a % 64 == 0 for a, _ in spans) and spans[-1][1] <= total
+    assert all(e <= s for (_, e), (s, _) in zip(spans, spans[1:]))
+    names = ("attn.c_attn.weight", "attn.c_proj.weight", "mlp.c_fc.weight", "mlp.c_proj.weight", "ln_1.weight",
+             "ln_1.bias", "attn.c_attn.bias", "attn.c_proj.bias", "ln_2.weight", "ln_2.bias", "mlp.c_fc.bias",
+             "mlp.c_proj.bias")
+    assert len(numbers) == 18
+    for i in range(3):
+        for n, o in zip(names, numbers[6:]):
+            key = f"transformer.h.{i}.{n}"
+            assert (o == -1) == (key not in off)
+            if o >= 0:
+                assert numbers[2] + i * numbers[3] + o == off[key]
+
+
+def test_only_plain_models_take_the_decode_kernel():
+    plain = _model()
+    assert decode.plain_model(plain) and decode.plain_model(plain.bfloat16())
+    assert not decode.supports(plain, torch.zeros(1, 3, dtype=torch.int64))  # not on a GPU
+
+    def changed(edit, **kw):
+        m = _model(**kw)
+        edit(m)
+        return decode.plain_model(m)
+
+    class Own(nn.Linear):
+        pass
+
+    assert not changed(lambda m: m.register_forward_hook(lambda *a: None))
+    assert not changed(lambda m: m.transformer.h[1].mlp.register_forward_pre_hook(lambda *a: None))
+    assert not changed(lambda m: setattr(m.transformer.h[0].attn, "c_proj", Own(128, 128)))
+    assert not changed(lambda m: setattr(m.lm_head, "weight", nn.Parameter(m.lm_head.weight.detach().clone())))
+    assert not changed(lambda m: setattr(m.transformer.ln_f, "eps", 1e-6))
+    assert not changed(lambda m: setattr(m.transformer.h[0].attn, "num_heads", 1))
+    assert not changed(lambda m: m.transformer.h[0].double())
+    assert not changed(lambda m: m.half())
+    assert not changed(lambda m: m.transformer.wpe.__setattr__("weight", nn.Parameter(torch.zeros(41, 128))))
+    assert not changed(lambda m: setattr(m.transformer.h[0].mlp.c_fc, "bias", None))
+    assert not changed(lambda m: setattr(m.transformer.h[0].mlp.c_fc, "weight",
+                                         nn.Parameter(torch.zeros(128, 512).t())))
+    assert not changed(lambda m: m.train(), dropout=0.1)
+    assert changed(lambda m: m.train()) and changed(lambda m: None, dropout=0.1)
+
+
+def _general(m, X):
+    """Logits after each prompt prefix, through the module's forward."""
+    return torch.stack([m(X[:, :t][:, -m.config.block_size:])[0][:, -1].float() for t in range(1, X.shape[1] + 1)], 1)
+
+
+# widths below one row per SM up to the widest, batches of one launch and of several, every kind of
+# remainder in vocabulary and length; several key ranges per head (one sequence, long context)
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,layers,vocab,block,B,T,ln_bias,bf16", [
+    (1, 1, 5, 9, 1, 9, True, False), (2, 2, 101, 40, 3, 12, False, False), (12, 2, 50257, 64, 8, 5, False, False),
+    (12, 2, 1000, 700, 1, 650, True, False), (25, 2, 50304, 300, 4, 270, False, True),
+    (32, 1, 777, 1024, 8, 530, True, False), (6, 3, 65, 128, 11, 100, True, True)])
+def test_decode_matches_the_forward_pass(heads, layers, vocab, block, B, T, ln_bias, bf16):
+    m = _model(heads, layers, vocab, block, ln_bias)
+    X = torch.randint(0, vocab, (B, T), generator=torch.Generator().manual_seed(1))
+    oracle = copy.deepcopy(m).double()
+    m = m.cuda().bfloat16() if bf16 else m.cuda()
+    if bf16:
+        oracle = copy.deepcopy(m).cpu().double()
+    n = min(T, 6)  # positions compared: the last six (the first ones of short prompts)
+    Xc = X.cuda()
+    with torch.inference_mode():
+        assert decode.supports(m, Xc)
+        s = decode.DecodeSession(m, B, T)
+        s.prefill(Xc[:, :T - n])
+        got = torch.stack([s.step(Xc[:, t], t).clone() for t in range(T - n, T)], 1).cpu().double()
+        mod = torch.stack([m(Xc[:, :t + 1])[0][:, -1].float() for t in range(T - n, T)], 1).cpu().double()
+        ref = torch.stack([oracle(X[:, :t + 1])[0][:, -1] for t in range(T - n, T)], 1)
+    scale = ref.norm()
+    e_got, e_mod = (got - ref).norm() / scale, (mod - ref).norm() / scale
+    # both round activations to bf16 at the same places, so their errors are two draws of one size
+    assert e_got <= 1.3 * e_mod + 1e-3, (float(e_got), float(e_mod))
+
+
+@pytest.mark.gpu
+def test_generate_past_the_context_window_and_sampling_seeds():
+    m = _model(heads=2, layers=2, vocab=101, block=24).cuda()
+    X = torch.randint(0, 101, (2, 20), generator=torch.Generator().manual_seed(2)).cuda()
+    for kw in ({"top_k": 1}, {"temperature": 0.9, "top_k": 7}):
+        torch.manual_seed(3)
+        out = m.generate(X, 12, **kw)
+        handle = m.register_forward_hook(lambda *a: None)  # the general path
+        torch.manual_seed(3)
+        want = m.generate(X, 12, **kw)
+        handle.remove()
+        assert out.shape == (2, 32) and torch.equal(out[:, :20], X) and out.dtype == want.dtype
+        assert (out == want).float().mean() > 0.9  # a near-tie may fall the other way after rounding
+    torch.manual_seed(3)
+    again = m.generate(X, 12, temperature=0.9, top_k=7)
+    torch.manual_seed(3)
+    assert torch.equal(again, m.generate(X, 12, temperature=0.9, top_k=7))
+    g = torch.Generator("cuda").manual_seed(4)
+    assert m.generate(X.int(), 2, generator=g).shape == (2, 22) and m.generate(X, 0) is X
+
+
+# the top-k select: values that crowd into one first digit, ties, both signs of zero, -inf, one row in
+# shared memory and one too long for it
+@pytest.mark.gpu
+@pytest.mark.parametrize("V", (1, 33, 1000, 50257, 56321))
+def test_top_k_keeps_what_the_sort_keeps(V):
+    from zero_to_hero_b200.ops.sampling import sample_next, sample_topk_native
+
+    g = torch.Generator().manual_seed(V)
+    rows = torch.stack((torch.randn(V, generator=g), 3 + 0.01 * torch.randn(V, generator=g), -100 - torch.rand(V, generator=g),
+                        torch.randint(-2, 3, (V,), generator=g) * 1.0, torch.full((V,), -torch.inf)))
+    rows[3][rows[3] == 0] *= -1.0  # some -0.0 beside 1.0 and 2.0
+    rows[4, V // 2] = -3.0
+    for k in (1, 2, 7, V - 1, V, None):
+        if k is not None and not 0 < k <= V:
+            continue
+        many = rows.repeat(64, 1).cuda()
+        column = torch.zeros(many.shape[0], 3, dtype=torch.int64, device="cuda")
+        ids = sample_topk_native(many, 1.0, k, seed=5, out=column[:, 1])
+        assert torch.equal(ids[:, 0], column[:, 1]) and not column[:, (0, 2)].any()
+        assert torch.equal(ids, sample_topk_native(many, 1.0, k, seed=5))
+        low = rows.topk(k if k else V).values[:, -1].repeat(64)
+        picked = many.cpu().gather(1, ids.cpu()).squeeze(1)
+        assert (picked >= low).all() and (picked > -torch.inf).all()
+        if k == 1:
+            assert torch.equal(picked, low)
+    assert sample_next(rows[:2].cuda(), out=column[:2, 0]).shape == (2, 1)

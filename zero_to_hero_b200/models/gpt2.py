@@ -178,9 +178,15 @@ class GPT2(nn.Module):
     def generate(self, X: torch.Tensor, max_new_tokens: int, temperature: float = 1.0,
                  top_k: int | None = None, generator: torch.Generator | None = None):
         """Autoregressive sampling (nn/gpt2/modules.py:121-137): crop to block_size, scale the
-        last-position logits by 1/temperature, optional top-k, softmax, multinomial."""
+        last-position logits by 1/temperature, optional top-k, softmax, multinomial. On a GPU keys and
+        values are cached (ops/decode.py) where the model is one the decode kernel computes."""
+        from ..ops import decode
         from ..ops.sampling import sample_next
 
+        if max_new_tokens > 0 and decode.supports(self, X):
+            out = decode.generate(self, X, max_new_tokens, temperature, top_k, generator)
+            if out is not None:
+                return out
         for _ in range(max_new_tokens):
             ctx = X if X.size(1) <= self.config.block_size else X[:, -self.config.block_size:]
             logits, _ = self(ctx)
