@@ -1,0 +1,98 @@
+"""The transformer block as one autograd node: which blocks take it (CPU) and its results (GPU)."""
+import copy
+
+import pytest
+import torch
+import torch.nn as nn
+
+from zero_to_hero_b200.config import ModelConfig
+from zero_to_hero_b200.models.gpt import GPTLM
+from zero_to_hero_b200.models.gpt2 import GPT2
+
+
+def _gpt2(heads=2, layers=2, vocab=96, block=64, ln_bias=True, dropout=0.0):
+    torch.manual_seed(0)
+    return GPT2(ModelConfig(vocab_size=vocab, block_size=block, emb_dim=64 * heads, num_heads=heads, num_layers=layers,
+                            dropout=dropout, ln_bias=ln_bias))
+
+
+def _char(heads=2, layers=2, vocab=65, block=64, dropout=0.0):
+    torch.manual_seed(0)
+    return GPTLM(vocab, block, 64 * heads, layers, heads, dropout)
+
+
+def test_only_plain_blocks_are_fused():
+    def gpt2(edit, **kw):
+        m = _gpt2(**kw)
+        edit(m.transformer.h[0])
+        return m.transformer.h[0]._parts() is not None
+
+    def char(edit, **kw):
+        m = _char(**kw)
+        edit(m.blocks[0])
+        return m.blocks[0]._parts() is not None
+
+    class Own(nn.Linear):
+        pass
+
+    for case, inner in ((gpt2, lambda b: b.mlp), (char, lambda b: b.ff)):
+        assert case(lambda b: None) and case(lambda b: b.eval(), dropout=0.1) and not case(lambda b: None, dropout=0.1)
+        assert case(lambda b: b.register_forward_hook(lambda *a: None))  # the block is still called as a module
+        assert not case(lambda b: inner(b).register_forward_hook(lambda *a: None))
+        assert not case(lambda b: inner(b).register_full_backward_hook(lambda *a: None))
+        assert not case(lambda b: b.attn.register_forward_pre_hook(lambda *a: None))
+        assert not case(lambda b: setattr(b.attn, "forward", lambda x: x))
+    assert not gpt2(lambda b: setattr(b.attn, "c_attn", Own(128, 384)))
+    assert not char(lambda b: setattr(b.attn.heads[1], "key", Own(128, 64, bias=False)))
+    assert not char(lambda b: setattr(b.ff.ff, "1", nn.GELU()))
+    from zero_to_hero_b200.ops import block as FB
+    assert not FB.usable(torch.zeros(1, 2, 128, dtype=torch.bfloat16), 2, [torch.zeros(128)])  # not on a GPU
+    assert not FB.shaped([torch.zeros(3), None], ((3,), (3, 3))) and FB.shaped([torch.zeros(3), None], ((3,), (3,)))
+
+
+def _grads(model, X, Y):
+    model.zero_grad(set_to_none=True)
+    logits, loss = model(X, Y)
+    loss.backward()
+    return logits.detach().double().cpu(), [p.grad.double().cpu() for p in model.parameters()]
+
+
+# one token, a whole and a part of a 32-row group, several tiles; one head up to a wide block; tied and untied
+# vocabularies of both kinds; fp32 and bf16 parameters; LayerNorm with and without bias
+@pytest.mark.gpu
+@pytest.mark.parametrize("make,B,T,kw,bf16", [
+    (_gpt2, 1, 1, {"heads": 1}, False), (_gpt2, 2, 64, {"ln_bias": False}, False), (_gpt2, 3, 41, {"vocab": 97}, False),
+    (_gpt2, 4, 300, {"heads": 12, "block": 512}, False), (_gpt2, 2, 50, {"heads": 3}, True),
+    (_char, 1, 3, {"heads": 1}, False), (_char, 5, 63, {}, False), (_char, 8, 256, {"heads": 6, "block": 256}, False)])
+def test_block_matches_the_single_ops(make, B, T, kw, bf16):
+    m = make(**kw)
+    vocab = m.config.vocab_size if make is _gpt2 else 65
+    g = torch.Generator().manual_seed(B * T)
+    X, Y = (torch.randint(0, vocab, (B, T), generator=g) for _ in range(2))
+    m = m.bfloat16() if bf16 else m
+    oracle = copy.deepcopy(m).double()
+    m = m.cuda()
+    blocks = m.transformer.h if make is _gpt2 else m.blocks
+    assert all(b._parts() is not None for b in blocks)
+    ref = _grads(oracle, X, Y)
+    got = _grads(m, X.cuda(), Y.cuda())
+    handles = [b.attn.register_forward_hook(lambda *a: None) for b in blocks]  # the single ops
+    single = _grads(m, X.cuda(), Y.cuda())
+    for h in handles:
+        h.remove()
+
+    def off(r):
+        scale = torch.sqrt(sum(v.square().sum() for v in ref[1]))
+        return (float((r[0] - ref[0]).norm() / ref[0].norm()),
+                float(torch.sqrt(sum((a - b).square().sum() for a, b in zip(r[1], ref[1]))) / scale))
+
+    # the same rounding points, so two draws of one error; 2e-3 is a single bf16 rounding
+    for a, b in zip(off(got), off(single)):
+        assert a <= 1.3 * b + 2e-3, (off(got), off(single))
+    frozen = [p for b in blocks for p in b.parameters() if p.dim() >= 2][:2]
+    for p in frozen:
+        p.requires_grad_(False)
+    m.zero_grad(set_to_none=True)
+    m(X.cuda(), Y.cuda())[1].backward()
+    assert all(p.grad is None for p in frozen)
+    assert all(p.grad is not None for p in m.parameters() if p.requires_grad)

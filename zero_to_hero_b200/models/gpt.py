@@ -18,7 +18,9 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops import block as FB
 from ..ops import functional as Z
+from ..ops.block import plain_modules
 from ..ops.sampling import sample_next
 
 
@@ -102,7 +104,37 @@ class Block(nn.Module):
         self.ln2 = LayerNorm(emb_dim)
         self.ff = FeedForward(emb_dim, dropout)
 
+    def _parts(self):
+        """(parameters of `ops.block.block`) when calling the parts of this block would run exactly their
+        classes' forwards without dropout, else None."""
+        attn, ff = self.attn, self.ff
+        seq = ff.ff
+        known = [(self.ln1, LayerNorm), (self.ln2, LayerNorm), (attn, MultiHeadAttention), (attn.proj, nn.Linear),
+                 (attn.heads, nn.ModuleList), (ff, FeedForward), (seq, nn.Sequential)]
+        if len(seq) != 5 or len(attn.heads) != attn.num_heads:
+            return None
+        known += list(zip(seq, (nn.Linear, nn.ReLU, nn.Dropout, nn.Linear, nn.Dropout)))
+        known += [(h, Head) for h in attn.heads]
+        known += [(m, nn.Linear) for h in attn.heads for m in (h.query, h.key, h.value)]
+        if not plain_modules(known) or (attn.training and attn.p > 0.0) or \
+                any(d.training and d.p > 0.0 for d in (seq[2], seq[4])):
+            return None
+        if any(m.bias is not None for h in attn.heads for m in (h.query, h.key, h.value)):
+            return None
+        qkv = [getattr(h, n).weight for n in ("query", "key", "value") for h in attn.heads]
+        return ((self.ln1.weight, self.ln1.bias), None, (attn.proj.weight, attn.proj.bias),
+                (self.ln2.weight, self.ln2.bias), (seq[0].weight, seq[0].bias), (seq[3].weight, seq[3].bias), qkv)
+
     def forward(self, X):
+        if X.is_cuda:
+            parts = self._parts()
+            if parts is not None:
+                flat = [t for p in parts for t in (p if isinstance(p, (tuple, list)) else (p,))]
+                C, H = X.shape[-1], self.attn.num_heads
+                shapes = ((C,), (C,), None, (C, C), (C,), (C,), (C,), (4 * C, C), (4 * C,), (C, 4 * C), (C,))
+                shapes += ((64, C),) * (3 * H)
+                if FB.usable(X, H, flat) and FB.shaped(flat, shapes):
+                    return FB.block(X, H, "relu", self.ln1.eps, self.ln2.eps, *parts)
         X = X + self.attn(self.ln1(X)).to(X.dtype)
         X = X + self.ff(self.ln2(X)).to(X.dtype)
         return X

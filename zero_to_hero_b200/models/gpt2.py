@@ -22,8 +22,10 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..config import ModelConfig
+from ..ops import block as FB
 from ..ops import dropout as D
 from ..ops import functional as Z
+from ..ops.block import plain_modules
 
 
 class LayerNorm(nn.Module):
@@ -108,7 +110,27 @@ class Block(nn.Module):
         self.ln_2 = LayerNorm(cfg.emb_dim, cfg.ln_bias)
         self.mlp = MLP(cfg)
 
+    def _parts(self):
+        """(parameters of `ops.block.block`) when calling the parts of this block would run exactly their
+        classes' forwards without dropout, else None."""
+        attn, mlp = self.attn, self.mlp
+        known = ((self.ln_1, LayerNorm), (self.ln_2, LayerNorm), (attn, Attention), (mlp, MLP), (attn.c_attn, nn.Linear),
+                 (attn.c_proj, nn.Linear), (mlp.c_fc, nn.Linear), (mlp.c_proj, nn.Linear))
+        if not plain_modules(known) or (attn.training and attn.dropout > 0.0) or (mlp.training and mlp.dropout > 0.0):
+            return None
+        return ((self.ln_1.weight, self.ln_1.bias), attn.c_attn.bias, (attn.c_proj.weight, attn.c_proj.bias),
+                (self.ln_2.weight, self.ln_2.bias), (mlp.c_fc.weight, mlp.c_fc.bias),
+                (mlp.c_proj.weight, mlp.c_proj.bias), (attn.c_attn.weight,))
+
     def forward(self, x, cdrop=None):
+        if x.is_cuda:
+            parts = self._parts()
+            if parts is not None:
+                flat = [t for p in parts for t in (p if isinstance(p, tuple) else (p,))]
+                C = x.shape[-1]
+                shapes = ((C,), (C,), (3 * C,), (C, C), (C,), (C,), (C,), (4 * C, C), (4 * C,), (C, 4 * C), (C,), (3 * C, C))
+                if FB.usable(x, self.attn.num_heads, flat) and FB.shaped(flat, shapes):
+                    return FB.block(x, self.attn.num_heads, "gelu_tanh", self.ln_1.eps, self.ln_2.eps, *parts)
         x = self.attn(self.ln_1(x), x, cdrop)  # pre-norm; the residual add is fused into the projection
         x = self.mlp(self.ln_2(x), x, cdrop)
         return x

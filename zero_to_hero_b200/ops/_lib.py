@@ -65,6 +65,16 @@ def stream_ptr() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+# The same as plain numbers, for functions whose argtypes are declared (a kernel launch from Python passes
+# half a dozen pointers; the ctypes objects cost more than the call).
+def address(t: torch.Tensor | None) -> int | None:
+    return None if t is None else t.data_ptr()
+
+
+def raw_stream() -> int:
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
 _status: dict[int, torch.Tensor] = {}
 
 

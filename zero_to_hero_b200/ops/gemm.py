@@ -11,10 +11,11 @@ from . import _lib
  EPI_MUL_AUX, EPI_SLICE_STORE) = range(9)
 
 _configured = False
+_entry = None  # z2h_gemm_bf16_ex, once its types are declared
 
 
 def _fn():
-    global _configured
+    global _configured, _entry
     lib = _lib.cuda_lib()
     if not _configured:
         lib.z2h_gemm_fold_slices.restype = ctypes.c_int
@@ -32,6 +33,7 @@ def _fn():
             ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p,
         ]
         _configured = True
+        _entry = lib.z2h_gemm_bf16_ex
     return lib.z2h_gemm_bf16_ex
 
 
@@ -55,23 +57,22 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = Fa
     `out`, `split_k == 1` and M, N multiples of 32.
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-    assert a.stride(-1) == 1 and b.stride(-1) == 1 and out.stride(-1) == 1
-    M, N = out.shape
-    K = a.shape[0] if a_mn else a.shape[1]
-    assert (a.shape[1] if a_mn else a.shape[0]) == M, (a.shape, out.shape, a_mn)
-    assert (b.shape[1] if b_mn else b.shape[0]) == N, (b.shape, out.shape, b_mn)
-    assert (b.shape[0] if b_mn else b.shape[1]) == K
+    (M, N), (a0, a1), (b0, b1) = out.shape, a.shape, b.shape
+    (lda, sa), (ldb, sb), (ldc, sc) = a.stride(), b.stride(), out.stride()
+    assert sa == 1 and sb == 1 and sc == 1
+    m, K = (a1, a0) if a_mn else (a0, a1)
+    n, k = (b1, b0) if b_mn else (b0, b1)
+    assert m == M and n == N and k == K, (a.shape, b.shape, out.shape, a_mn, b_mn)
     out_fp32 = out.dtype == torch.float32
     if colsum is not None:
         assert colsum.dtype == torch.float32 and colsum.numel() == N and colsum.is_contiguous()
     aux = aux_out if aux_out is not None else aux_in
-    rc = _fn()(
-        _lib.ptr(a), int(a_mn), a.stride(0), _lib.ptr(b), int(b_mn), b.stride(0),
-        _lib.ptr(out), out.stride(0), int(out_fp32), M, N, K, epi, split_k,
-        _lib.ptr(bias), _lib.ptr(residual), residual.stride(0) if residual is not None else 0,
-        _lib.ptr(aux_out), _lib.ptr(aux_in), aux.stride(0) if aux is not None else 0,
-        _lib.ptr(_lib.status_word(out.device)), max_ctas, _lib.ptr(colsum), int(slice_stride),
-        _lib.stream_ptr())
+    address = _lib.address
+    rc = (_entry or _fn())(
+        a.data_ptr(), int(a_mn), lda, b.data_ptr(), int(b_mn), ldb, out.data_ptr(), ldc, int(out_fp32), M, N, K, epi,
+        split_k, address(bias), address(residual), residual.stride(0) if residual is not None else 0, address(aux_out),
+        address(aux_in), aux.stride(0) if aux is not None else 0, _lib.status_word(out.device).data_ptr(), max_ctas,
+        address(colsum), int(slice_stride), _lib.raw_stream())
     if rc != 0:
         raise RuntimeError(f"z2h_gemm_bf16 failed with code {rc} for M={M} N={N} K={K}")
     return out
@@ -83,7 +84,7 @@ def fold_slices(slices: torch.Tensor, num_slices: int, dst: torch.Tensor) -> Non
     assert slices.dtype == torch.float32 and dst.dtype == torch.float32 and dst.is_contiguous()
     assert slices.numel() >= num_slices * n and n % 4 == 0
     _fn()
-    rc = _lib.cuda_lib().z2h_gemm_fold_slices(_lib.ptr(slices), num_slices, n, _lib.ptr(dst), _lib.stream_ptr())
+    rc = _lib.cuda_lib().z2h_gemm_fold_slices(_lib.address(slices), num_slices, n, _lib.address(dst), _lib.raw_stream())
     if rc != 0:
         raise RuntimeError(f"z2h_gemm_fold_slices failed with code {rc}")
 

@@ -7,12 +7,13 @@ autograd-aware, module-level API lives in `zero_to_hero_b200.ops.functional`.
 from __future__ import annotations
 
 import ctypes
+import itertools
 from ctypes import c_int, c_longlong, c_float, c_void_p
 
 import torch
 
 from . import _lib
-from ._lib import ptr, stream_ptr
+from ._lib import address as ptr, raw_stream as stream_ptr
 
 _sigs = {
     "z2h_layernorm_fwd": [c_void_p] * 6 + [c_int, c_int, c_float, c_void_p],
@@ -37,6 +38,9 @@ _sigs = {
     "z2h_ce_bwd": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, c_longlong, c_int, c_int, c_int,
                    c_int, c_void_p],
     "z2h_compact_rows": [c_void_p, c_longlong, c_void_p, c_int, c_int, c_void_p],
+    "z2h_relu": [c_void_p, c_longlong, c_void_p],
+    "z2h_relu_bwd": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
+    "z2h_pack_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p],
     "z2h_gelu_bwd": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "z2h_reduce_sum": [c_void_p, c_int, c_float, c_void_p, c_int, c_void_p],
     "z2h_gradnorm_partials": [c_void_p, c_longlong, c_void_p, c_void_p],
@@ -157,6 +161,29 @@ def gelu_bwd(dy, pre, dx, db=None):
     """dx = dy * gelu_tanh'(pre) over tight bf16 [M, N]; `db` (fp32 [N]) += column sums of dx."""
     M, N = pre.shape
     _check(_f("z2h_gelu_bwd")(ptr(dy), ptr(pre), ptr(dx), ptr(db), M, N, stream_ptr()), "gelu_bwd")
+
+
+def relu_(x):
+    """In place over a contiguous bf16 tensor whose size is a multiple of 8."""
+    _check(_f("z2h_relu")(ptr(x), x.numel(), stream_ptr()), "relu")
+
+
+def relu_bwd(dy, out, dx, db=None):
+    """dx = dy where out > 0, else 0, over tight bf16 [M, N]; `db` (fp32 [N]) += column sums of dx."""
+    M, N = out.shape
+    _check(_f("z2h_relu_bwd")(ptr(dy), ptr(out), ptr(dx), ptr(db), M, N, stream_ptr()), "relu_bwd")
+
+
+def pack_bf16(tensors, sizes):
+    """bf16 copies of contiguous, 16-byte aligned tensors of one type (fp32 or bf16), whose sizes are multiples
+    of 64, one after the other in one buffer, by one launch (per 128 tensors)."""
+    n = len(tensors)
+    at = list(itertools.accumulate(sizes, initial=0))
+    flat = torch.empty(at[-1], device=tensors[0].device, dtype=torch.bfloat16)
+    _check(_f("z2h_pack_bf16")((c_void_p * n)(*[t.data_ptr() for t in tensors]), (c_longlong * n)(*at[:n]),
+                               (c_longlong * n)(*sizes), n, int(tensors[0].dtype == torch.float32), ptr(flat),
+                               stream_ptr()), "pack_bf16")
+    return flat
 
 
 def reduce_sum(x, out, scale=1.0, accumulate=False):
