@@ -42,7 +42,71 @@ dropout_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
   }
 }
 
+// The same over a matrix, with the column sums of what is stored added to db: the dropped gradient of a
+// projection's output and that projection's bias gradient in one pass (bound by memory: 4 bytes an element
+// instead of 4 + 2). A CTA takes 256 columns of a slab of rows, one row per warp.
+__global__ void __launch_bounds__(256)
+dropout_colsum_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, float* __restrict__ db,
+                      int M, int N, int rows_per_slab, float p, const unsigned long long* __restrict__ seed_ptr,
+                      uint32_t site) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float sums[8][256];
+  const DropoutSpec d = make_dropout_spec(seed_ptr, site, p);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = blockIdx.x * 256 + lane * 8;
+  const int r1 = min(M, (int)(blockIdx.y + 1) * rows_per_slab);
+  float s[8] = {};
+  if (col < N) {
+#pragma unroll 4
+    for (int r = blockIdx.y * rows_per_slab + warp; r < r1; r += 8) {
+      const long long at = (long long)r * N + col;
+      const uint4 u = *reinterpret_cast<const uint4*>(x + at);
+      const uint32_t* w = &u.x;
+      const uint32_t m0 = dropout_word(d.seed_lo, d.seed_hi, (unsigned long long)at / 4);
+      const uint32_t m1 = dropout_word(d.seed_lo, d.seed_hi, (unsigned long long)at / 4 + 1);
+      uint4 o;
+      uint32_t* ow = &o.x;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = unpack_bf16x2(w[j]);
+        const uint32_t m = j < 2 ? m0 : m1;
+        const int e = (2 * j) & 3;
+        ow[j] = pack_bf16x2(dropout_keep(m, e, d.threshold) ? f.x * d.scale : 0.f,
+                            dropout_keep(m, e + 1, d.threshold) ? f.y * d.scale : 0.f);
+        const float2 q = unpack_bf16x2(ow[j]);
+        s[2 * j] += q.x;
+        s[2 * j + 1] += q.y;
+      }
+      *reinterpret_cast<uint4*>(out + at) = o;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sums[warp][lane * 8 + j] = s[j];
+  __syncthreads();
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c < N) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += sums[k][threadIdx.x];
+    atomicAdd(db + c, t);
+  }
+}
+
 }  // namespace
+
+int dropout_colsum(const void* x, void* out, float* db, int M, int N, float p, const unsigned long long* seed_ptr,
+                   unsigned int site, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (N % 8 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15)) return 1;
+  if (!(p >= 0.f) || p >= 1.f) return 1;
+  const int cols = (N + 255) / 256;
+  int slabs = (8 * sm_count_current_device() + cols - 1) / cols, rows = (M + slabs - 1) / slabs;
+  if (rows < 32) rows = 32;  // at least four rows per warp
+  slabs = (M + rows - 1) / rows;
+  launch_kernel(dropout_colsum_kernel, dim3(cols, slabs), dim3(256), 0, stream, true, (const __nv_bfloat16*)x,
+                (__nv_bfloat16*)out, db, M, N, rows, p, seed_ptr, site);
+  return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
 
 int dropout_apply(const void* x, const void* residual, void* out, long long n, float p,
                   const unsigned long long* seed_ptr, unsigned int site, cudaStream_t stream) {
@@ -65,4 +129,9 @@ int dropout_apply(const void* x, const void* residual, void* out, long long n, f
 extern "C" int z2h_dropout_apply(const void* x, const void* residual, void* out, long long n, float p,
                                  const unsigned long long* seed_ptr, unsigned int site, void* stream) {
   return z2h::dropout_apply(x, residual, out, n, p, seed_ptr, site, (cudaStream_t)stream);
+}
+// out = dropout(x) over a tight [M, N], db (fp32 [N]) += column sums of out
+extern "C" int z2h_dropout_colsum(const void* x, void* out, float* db, int M, int N, float p,
+                                  const unsigned long long* seed_ptr, unsigned int site, void* stream) {
+  return z2h::dropout_colsum(x, out, db, M, N, p, seed_ptr, site, (cudaStream_t)stream);
 }

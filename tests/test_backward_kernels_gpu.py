@@ -88,3 +88,17 @@ def test_ordered_embedding_gradient(B, T, C, V):
         dwte, dwpe = torch.zeros(V, C, device="cuda"), torch.zeros(T, C, device="cuda")
         N.embed_bwd(idx.to(dtype).cuda(), dx.cuda(), dwte, dwpe, B, T, ordered=True)
         assert torch.equal(dwte.cpu(), want)
+
+
+@pytest.mark.parametrize("M,N", [(1, 8), (33, 264), (4099, 768)])
+def test_dropout_with_column_sums(M, N):
+    from zero_to_hero_b200.ops import native
+
+    x = torch.randn(M, N, generator=torch.Generator().manual_seed(M)).bfloat16().cuda()
+    seed = torch.tensor([7], device="cuda")
+    want, out = torch.empty_like(x), torch.empty_like(x)
+    native.dropout_apply(x, want, 0.2, seed, 5)
+    db = torch.ones(N, device="cuda")
+    native.dropout_colsum(x, out, db, 0.2, seed, 5)
+    assert torch.equal(out, want)
+    assert torch.allclose(db.double(), 1 + want.double().sum(0), rtol=1e-4, atol=1e-4 * M ** 0.5)

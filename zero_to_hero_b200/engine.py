@@ -292,7 +292,9 @@ class GPT2TrainEngine:
         self.micro_steps_done = 0
         if self.drop_p > 0.0:
             self.drop_tmp = buf(M, C)  # projection output before dropout + residual
-            self.d_drop = buf(M, C)    # gradient of that output
+            # gradient of that output; one for the MLP and one for attention, because a weight gradient on
+            # the side stream may still read the one while the chain writes the other
+            self.d_drop = [buf(M, C), buf(M, C)]
         self.d_4c = buf(M, 4 * C)
         self.d_qkv = buf(M, 3 * C)
         self.dq_copies = N.flash_bwd_copies(B, T, H) if self.cfg.train.deterministic else 1
@@ -463,7 +465,7 @@ class GPT2TrainEngine:
         G.gemm(logits_v, w("transformer.wte.weight"), self.d_c, b_mn=True)
         self._n += 1
         self._wgrad(logits_v, self.xf, "transformer.wte.weight")  # fills the machine by itself: main stream
-        self._overlap = bool(self.cfg.train.overlap_wgrad) and pd == 0.0
+        self._overlap = bool(self.cfg.train.overlap_wgrad)
         self._side_done = []
         R = [self.d_resid, self.d_resid_alt if self._overlap else self.d_resid]
         cur = 0  # R[cur] holds the residual-stream gradient
@@ -471,6 +473,18 @@ class GPT2TrainEngine:
         # output that was added into it, so the LayerNorm backward that produces it also sums its
         # columns into that projection's bias gradient (no separate pass over it).
         fuse_db = pd == 0.0
+
+        def drop_gradient(dy, out, site, bias):
+            # gradient of a projection's output: the residual-stream gradient through the mask, and its
+            # column sums, the bias gradient (added with atomics, so the reproducible mode sums apart)
+            if self.deterministic:
+                N.dropout_apply(dy, out, pd, seed, site)
+            else:
+                N.dropout_colsum(dy, out, gw(bias), pd, seed, site)
+            self._n += 1
+            return out
+
+        separate_db = pd > 0.0 and self.deterministic
         N.layernorm_bwd(self.d_c, self.resid[L], w("transformer.ln_f.weight"), self.stats_f[0],
                         self.stats_f[1], None, R[cur], gw("transformer.ln_f.weight"),
                         glnb("transformer.ln_f.bias"), self.ln_scratch,
@@ -483,13 +497,11 @@ class GPT2TrainEngine:
             # dropout mask of the forward pass)
             dy = R[cur]
             if pd > 0.0:
-                N.dropout_apply(R[cur], self.d_drop, pd, seed, 3 + 3 * l)
-                dy = self.d_drop
-                self._n += 1
+                dy = drop_gradient(dy, self.d_drop[0], 3 + 3 * l, p + "mlp.c_proj.bias")
 
             def wg_mlp_proj(dy=dy, l=l, p=p):
                 self._wgrad(dy, self.act[l], p + "mlp.c_proj.weight")
-                if not fuse_db:
+                if separate_db:
                     N.colsum_bf16(dy, gw(p + "mlp.c_proj.bias"), ordered=self.deterministic,
                                   scratch=self._colsum_scratch)
 
@@ -521,13 +533,11 @@ class GPT2TrainEngine:
             # attention
             dy = R[cur]
             if pd > 0.0:
-                N.dropout_apply(R[cur], self.d_drop, pd, seed, 2 + 3 * l)
-                dy = self.d_drop
-                self._n += 1
+                dy = drop_gradient(dy, self.d_drop[1], 2 + 3 * l, p + "attn.c_proj.bias")
 
             def wg_attn_proj(dy=dy, l=l, p=p):
                 self._wgrad(dy, self.att[l], p + "attn.c_proj.weight")
-                if not fuse_db:
+                if separate_db:
                     N.colsum_bf16(dy, gw(p + "attn.c_proj.bias"), ordered=self.deterministic,
                                   scratch=self._colsum_scratch)
 
@@ -555,12 +565,12 @@ class GPT2TrainEngine:
                             self.ln_scratch,
                             dxsum=gw(f"transformer.h.{l - 1}.mlp.c_proj.bias") if fuse_db and l > 0 else None)
             cur = 1 - cur
-            # dgrad GEMMs, column-sum launches (the projection biases ride in the LayerNorm backward
-            # without dropout, the QKV bias in the attention kernels, the c_fc bias usually in its
+            # dgrad GEMMs, column-sum launches (the projection biases ride in the LayerNorm backward or in
+            # the dropout pass, the QKV bias in the attention kernels, the c_fc bias usually in its
             # GEMM), LN bwd (2 kernels each), flash bwd (3)
             # (reproducible mode without memory for copies of dQ: one attention launch per KV tile; plus the
             # QKV column sum)
-            self._n += 4 + (0 if fuse_db else 2) + (0 if fc_db_in_gemm else 1) + 2 * 2
+            self._n += 4 + (2 if separate_db else 0) + (0 if fc_db_in_gemm else 1) + 2 * 2
             self._n += (2 + (1 if self.dq_copies > 1 else (T + 127) // 128) + 1) if det else 3
             if reduce:
                 self._reduce_ready(l)

@@ -56,6 +56,7 @@ _sigs = {
                             c_void_p, c_void_p, c_void_p],
     "z2h_flash_bwd_dropout": [c_void_p] * 7 + [c_int, c_int, c_int, c_float, c_void_p, ctypes.c_uint,
                                                c_void_p, c_void_p],
+    "z2h_dropout_colsum": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p, ctypes.c_uint, c_void_p],
     "z2h_dropout_apply": [c_void_p, c_void_p, c_void_p, c_longlong, c_float, c_void_p, ctypes.c_uint,
                           c_void_p],
 }
@@ -310,3 +311,12 @@ def dropout_apply(x, out, drop_p: float, seed, site: int, residual=None):
         assert residual.is_contiguous() and residual.numel() == x.numel()
     _check(_f("z2h_dropout_apply")(ptr(x), ptr(residual), ptr(out), x.numel(), drop_p, ptr(seed), site,
                                    stream_ptr()), "dropout_apply")
+
+
+def dropout_colsum(x, out, db, drop_p: float, seed, site: int):
+    """out = dropout(x) over a contiguous bf16 [M, N] with the mask `dropout_apply` uses; `db` (fp32 [N])
+    += column sums of out."""
+    assert x.is_contiguous() and out.is_contiguous() and x.dtype == torch.bfloat16 and db.dtype == torch.float32
+    M, N = x.shape
+    _check(_f("z2h_dropout_colsum")(ptr(x), ptr(out), ptr(db), M, N, drop_p, ptr(seed), site, stream_ptr()),
+           "dropout_colsum")
