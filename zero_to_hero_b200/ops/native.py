@@ -6,6 +6,7 @@ autograd-aware, module-level API lives in `zero_to_hero_b200.ops.functional`.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import itertools
 from ctypes import c_int, c_longlong, c_float, c_void_p
@@ -38,6 +39,7 @@ _sigs = {
     "z2h_ce_bwd": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, c_longlong, c_int, c_int, c_int,
                    c_int, c_void_p],
     "z2h_compact_rows": [c_void_p, c_longlong, c_void_p, c_int, c_int, c_void_p],
+    "z2h_pdl_scope": [c_int],
     "z2h_relu": [c_void_p, c_longlong, c_void_p],
     "z2h_relu_bwd": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "z2h_pack_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p],
@@ -76,6 +78,16 @@ def _f(name: str):
 def _check(rc: int, name: str) -> None:
     if rc != 0:
         raise RuntimeError(f"{name} failed with code {rc} (1 bad argument, 2 tensor map, 3 launch)")
+
+
+@contextlib.contextmanager
+def pdl_scope(on: bool):
+    """Launches of this thread inside the block use programmatic dependent launch (csrc/common/launch.cuh)."""
+    before = _f("z2h_pdl_scope")(int(on))
+    try:
+        yield
+    finally:
+        _f("z2h_pdl_scope")(before)
 
 
 def _is64(t: torch.Tensor) -> int:
