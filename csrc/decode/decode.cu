@@ -61,9 +61,8 @@ struct Params {
   DecodeArgs a;
   int slots, slot_bytes, xs_stride, splits;  // a slot: slot_bytes of weights, kBiasBytes of biases
   // exchange buffers, 8 bytes a unit: two bf16 values (or one fp32) and the epoch
-  uint64_t *resid, *mid, *act;  // [batch][C / 2], [batch][C / 2], [batch][4C / 2]
-  uint64_t *qkv, *att;          // [batch][3C / 2], [batch][C / 2]
-  uint64_t* part;               // [batch][heads][splits][kPartFloats]
+  uint64_t *resid, *mid, *att, *act, *qkv;  // [batch][C / 2], act: 4C / 2, qkv: 3C / 2
+  uint64_t* part;                           // [batch][heads][splits][kPartFloats]
 };
 
 // How a matrix of n rows and K columns is cut for the ring: tiles of `rows` rows, `cols` columns a slot.
@@ -179,6 +178,11 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// One instance of the bounded wait for all its places.
+__device__ __noinline__ bool wait_for(Smem* sm, uint64_t* bar, uint32_t phase, int* status, int code) {
+  return mbar_wait_bounded(bar, phase, &sm->abort_flag, status, code);
+}
+
 // ---- producer (a warp) --------------------------------------------------------------------------
 struct Ring {
   int slot = 0;
@@ -197,8 +201,8 @@ struct Producer {
   const __nv_bfloat16* w;
 
   // lane 0 has the slot's transaction count armed on return
-  __device__ bool open(uint32_t bytes) {
-    const bool ok = mbar_wait_bounded(&sm->empty[st.slot], st.phase ^ 1, &sm->abort_flag, p.a.status, kTimeoutEmpty);
+  __device__ __noinline__ bool open(uint32_t bytes) {
+    const bool ok = wait_for(sm, &sm->empty[st.slot], st.phase ^ 1, p.a.status, kTimeoutEmpty);
     if (!__all_sync(0xffffffffu, ok)) return false;
     if ((threadIdx.x & 31) == 0) mbar_arrive_expect_tx(&sm->full[st.slot], bytes);
     __syncwarp();
@@ -211,7 +215,7 @@ struct Producer {
   __device__ uint8_t* at() const { return ring + (size_t)st.slot * (p.slot_bytes + kBiasBytes); }
 
   // bias < 0: none
-  __device__ bool matrix(Matrix which, long long offset, long long bias, int K) {
+  __device__ bool matrix(int which, long long offset, long long bias, int K) {
     const Share own = sm->share[which];
     const int lane = threadIdx.x & 31;
     for (int r = own.r0; r < own.r1; r += own.rows) {
@@ -253,7 +257,7 @@ struct Producer {
 // sequence exist). `bias`: where the biases lie in the packed buffer, < 0: there are none.
 template <typename Done>
 __device__ __forceinline__ void matvec(const Params& p, Smem* sm, const uint8_t* ring, const uint8_t* xs, Ring& st,
-                                       int& buf, Matrix which, int K, long long bias, Done done) {
+                                       int& buf, int which, int K, long long bias, Done done) {
   const Share own = sm->share[which];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int in_tile = (int)threadIdx.x >> 3, b = threadIdx.x & 7;
@@ -266,14 +270,14 @@ __device__ __forceinline__ void matvec(const Params& p, Smem* sm, const uint8_t*
     float acc[4][4] = {}, add = 0.f;  // four chains: a step's products do not wait for each other
     for (int k = 0; k < K; k += own.cols) {
       const int n = min(own.cols, K - k);
-      mbar_wait_bounded(&sm->full[st.slot], st.phase, &sm->abort_flag, p.a.status, kTimeoutFull);
+      wait_for(sm, &sm->full[st.slot], st.phase, p.a.status, kTimeoutFull);
       const uint8_t* slot = ring + (size_t)st.slot * (p.slot_bytes + kBiasBytes);
       if (k == 0 && bias >= 0 && mine)
         add = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(slot + p.slot_bytes)[((bias + r) & 7) + in_tile]);
       // rows that the tile does not have read its first one; nobody takes their sums
       const uint8_t* w0 = slot + t * 16 + (g < rows ? g : 0) * n * 2;
       const uint8_t* w1 = slot + t * 16 + (g + 8 < rows ? g + 8 : 0) * n * 2;
-#pragma unroll 2
+#pragma unroll 1
       for (int s = warp; s < n / 64; s += kWarps) {
         const uint4 a0f = *reinterpret_cast<const uint4*>(w0 + s * 128 + first);
         const uint4 a1f = *reinterpret_cast<const uint4*>(w1 + s * 128 + first);
@@ -366,7 +370,7 @@ __device__ __forceinline__ void layer_norm_rows(const Params& p, Smem* sm, const
   if (warp < p.a.batch) {
     uint8_t* row = xs + warp * p.xs_stride;
     float sum = 0.f, sq = 0.f;
-#pragma unroll 2
+#pragma unroll 1
     for (int c = lane * 8; c < C; c += 256) {
       const uint4 v = *reinterpret_cast<const uint4*>(row + c * 2);
       const uint32_t* u = &v.x;
@@ -379,7 +383,7 @@ __device__ __forceinline__ void layer_norm_rows(const Params& p, Smem* sm, const
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const float mean = sum / C;
-#pragma unroll 2
+#pragma unroll 1
     for (int c = lane * 8; c < C; c += 256) {
       const uint4 v = *reinterpret_cast<const uint4*>(row + c * 2);
       const uint32_t* u = &v.x;
@@ -392,9 +396,9 @@ __device__ __forceinline__ void layer_norm_rows(const Params& p, Smem* sm, const
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
     const float rstd = rsqrtf(sq / C + 1e-5f);
-    mbar_wait_bounded(&sm->full[st.slot], st.phase, &sm->abort_flag, p.a.status, kTimeoutFull);
+    wait_for(sm, &sm->full[st.slot], st.phase, p.a.status, kTimeoutFull);
     const uint8_t* norm = ring + (size_t)st.slot * (p.slot_bytes + kBiasBytes);
-#pragma unroll 2
+#pragma unroll 1
     for (int c = lane * 8; c < C; c += 256) {
       const uint4 v = *reinterpret_cast<const uint4*>(row + c * 2);
       const uint4 wv = *reinterpret_cast<const uint4*>(norm + c * 2);
@@ -485,14 +489,14 @@ __device__ __forceinline__ void attend(const Params& p, Smem* sm, int layer, uin
       mr = fmaxf(mr, __shfl_xor_sync(0xffffffffu, mr, 8));
       mr = fmaxf(mr, __shfl_xor_sync(0xffffffffu, mr, 16));
       if (mr > -INFINITY) {  // warp-uniform: this warp has keys in the round
-        const float mn = fmaxf(m, mr), keep = exp2f(m - mn);
+        const float mn = fmaxf(m, mr), keep = ex2_fast(m - mn);
         m = mn;
         l *= keep;
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] *= keep;
 #pragma unroll
         for (int i = 0; i < kKeysPerLane; ++i) {
-          const float e = exp2f(sc[i] - m);
+          const float e = ex2_fast(sc[i] - m);
           l += e;
           const uint32_t* w = &vv[i].x;
 #pragma unroll
@@ -519,11 +523,11 @@ __device__ __forceinline__ void attend(const Params& p, Smem* sm, int layer, uin
     consumer_sync();
     if (threadIdx.x < 64) {
       float M = -INFINITY, Lsum = 0.f, O = 0.f;
-#pragma unroll
+#pragma unroll 5
       for (int w = 0; w < kWarps; ++w) M = fmaxf(M, sm->att[w][0]);
-#pragma unroll
+#pragma unroll 5
       for (int w = 0; w < kWarps; ++w) {
-        const float mw = sm->att[w][0], f = mw > -INFINITY ? exp2f(mw - M) : 0.f;
+        const float mw = sm->att[w][0], f = mw > -INFINITY ? ex2_fast(mw - M) : 0.f;
         Lsum += sm->att[w][1] * f;
         O += sm->att[w][4 + threadIdx.x] * f;
       }
@@ -547,7 +551,6 @@ __device__ __forceinline__ void attend(const Params& p, Smem* sm, int layer, uin
 
 // xs[b] = attention output, folded from the key ranges' parts
 __device__ __forceinline__ void fold_attention(const Params& p, Smem* sm, uint8_t* xs, uint32_t epoch) {
-  if (p.splits == 1) return copy_rows(p, sm, xs, p.att, p.a.C, epoch);
   const int S = p.splits, quads = p.a.C / 4;
   for (int i = threadIdx.x; i < p.a.batch * quads; i += kConsumers) {
     int b = 0, c = i;
@@ -561,7 +564,7 @@ __device__ __forceinline__ void fold_attention(const Params& p, Smem* sm, uint8_
       gather(p, sm, 3, [&](int j) { return d + (j == 0 ? 0 : 2 + 2 * j + c % 64); }, epoch, v);
       const float ms = __uint_as_float(v[0].x);
       if (ms > -INFINITY) {
-        const float mn = fmaxf(m, ms), f = exp2f(m - mn), g = exp2f(ms - mn);
+        const float mn = fmaxf(m, ms), f = ex2_fast(m - mn), g = ex2_fast(ms - mn);
         m = mn;
         l = l * f + __uint_as_float(v[0].y) * g;
         o.x = o.x * f + __uint_as_float(v[1].x) * g;
@@ -576,14 +579,16 @@ __device__ __forceinline__ void fold_attention(const Params& p, Smem* sm, uint8_
   consumer_sync();
 }
 
-__device__ void consume(const Params& p, Smem* sm, const uint8_t* ring, uint8_t* xs) {
+// One loop over the phases of all layers with a single instance of each piece of code: laid out phase by
+// phase the kernel was 170 KB of code (65 KB now) and every phase began with instruction-cache misses (one
+// token of the 124M model 330 us, 248 so; of the 1.5B model for four sequences 2.4 and 1.7 ms).
+__device__ __forceinline__ void consume(const Params& p, Smem* sm, const uint8_t* ring, uint8_t* xs) {
   const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(p.a.weights);
   const DecodeLayout& lay = p.a.lay;
   const int C = p.a.C;
   const long long plane = (long long)p.a.batch * p.a.max_len * C;
   Ring st;
   int buf = 0;
-  uint32_t epoch = p.a.epoch_base;  // of the residual stream that a layer starts from
   // The matrices with C rows give every CTA the same rows each time: it keeps their values of the residual
   // stream for the next addition to it.
   const int own0 = sm->share[kProj].r0;
@@ -595,52 +600,69 @@ __device__ void consume(const Params& p, Smem* sm, const uint8_t* ring, uint8_t*
           __bfloat162float(W[lay.wte + tok * C + row]) + __bfloat162float(W[lay.wpe + (long long)p.a.pos * C + row])));
     }
   }
-  auto add_to_stream = [&](uint64_t* dst, uint32_t to) {
-    return [&p, sm, C, own0, dst, to](int r, int b, float y, bool mine) {
-      float* stream = &sm->stream[mine ? r - own0 : 0][b];
-      const __nv_bfloat16 v = __float2bfloat16(y + *stream);
-      if (mine) *stream = __bfloat162float(v);
-      put_pair(dst, C, r, b, v, mine, to);
-    };
-  };
-  auto norm_rows = [&](const uint64_t* src, uint32_t from, bool has_bias) {
-    if (src != nullptr) copy_rows(p, sm, xs, src, C, from);
-    layer_norm_rows(p, sm, ring, xs, st, has_bias);
-    st.advance(p.slots);
-  };
   if (int b = threadIdx.x >> 5; b < p.a.batch) {  // the tokens' embeddings
     const long long tok = token_of(p, b);
     for (int c = (threadIdx.x & 31) * 8; c < C; c += 256)
       *reinterpret_cast<uint4*>(xs + b * p.xs_stride + c * 2) = embed8(p, W, tok, c);
   }
   consumer_sync();
-  for (int l = 0; l < p.a.layers; ++l, epoch += kEpochsPerLayer) {
-    const long long base = lay.layer0 + l * lay.layer_stride;
-    __nv_bfloat16* kv = reinterpret_cast<__nv_bfloat16*>(p.a.kv) + 2 * l * plane;
-    norm_rows(l == 0 ? nullptr : p.resid, epoch, lay.o_ln1_b >= 0);
-    matvec(p, sm, ring, xs, st, buf, kQkv, C, base + lay.o_b_qkv, [&](int r, int b, float y, bool mine) {
-      const __nv_bfloat16 o = __float2bfloat16(y);
-      put_pair(p.qkv, 3 * C, r, b, o, mine, epoch + 1);
-      if (mine && r >= C) {  // for the steps to come; this one's attention reads the exchange
-        const int part = r >= 2 * C, c = r - (part + 1) * C;
-        kv[part * plane + ((long long)b * p.a.max_len + p.a.pos) * C + c] = o;
+  uint32_t epoch = p.a.epoch_base;  // of the phase's input
+  int which = kQkv, layer = 0;
+  while (true) {
+    // ---- input into xs
+    const int K = which == kFc2 ? 4 * C : C;
+    if (which == kProj) {
+      attend(p, sm, layer, epoch, epoch + 1);
+      ++epoch;
+    }
+    if (which == kProj && p.splits > 1) {
+      fold_attention(p, sm, xs, epoch);
+    } else if (layer > 0 || which != kQkv) {
+      copy_rows(p, sm, xs, which == kProj ? p.att : which == kFc ? p.mid : which == kFc2 ? p.act : p.resid, K, epoch);
+    }
+    if (which == kQkv || which == kFc || which == kHead) {
+      layer_norm_rows(p, sm, ring, xs, st, which == kQkv ? lay.o_ln1_b >= 0 : which == kFc ? lay.o_ln2_b >= 0 : lay.lnf_b >= 0);
+      st.advance(p.slots);
+    }
+    // ---- product
+    const long long o_bias = which == kQkv ? lay.o_b_qkv : which == kProj ? lay.o_b_proj : which == kFc ? lay.o_b_fc : lay.o_b_fc2;
+    const long long bias = which == kHead ? -1 : lay.layer0 + layer * lay.layer_stride + o_bias;
+    ++epoch;
+    matvec(p, sm, ring, xs, st, buf, which, K, bias, [&](int r, int b, float y, bool mine) {
+      if (which == kHead) {
+        if (mine) p.a.logits[(long long)b * p.a.vocab + r] = __bfloat162float(__float2bfloat16(y));
+        return;
+      }
+      if (which == kFc) y = gelu_tanh(y);
+      float* stream = nullptr;
+      if (which == kProj || which == kFc2) {
+        stream = &sm->stream[mine ? r - own0 : 0][b];
+        y += *stream;
+      }
+      const __nv_bfloat16 v = __float2bfloat16(y);
+      if (stream != nullptr && mine) *stream = __bfloat162float(v);
+      if (which == kQkv) {
+        put_pair(p.qkv, 3 * C, r, b, v, mine, epoch);
+        if (mine && r >= C) {  // for the steps to come; this one's attention reads the exchange
+          const int part = r >= 2 * C, c = r - (part + 1) * C;
+          reinterpret_cast<__nv_bfloat16*>(p.a.kv)[(2 * layer + part) * plane +
+                                                   ((long long)b * p.a.max_len + p.a.pos) * C + c] = v;
+        }
+      } else {
+        const int rows = which == kFc ? 4 * C : C;
+        put_pair(which == kProj ? p.mid : which == kFc ? p.act : p.resid, rows, r, b, v, mine, epoch);
       }
     });
-    attend(p, sm, l, epoch + 1, epoch + 2);
-    fold_attention(p, sm, xs, epoch + 2);
-    matvec(p, sm, ring, xs, st, buf, kProj, C, base + lay.o_b_proj, add_to_stream(p.mid, epoch + 3));
-    norm_rows(p.mid, epoch + 3, lay.o_ln2_b >= 0);
-    matvec(p, sm, ring, xs, st, buf, kFc, C, base + lay.o_b_fc, [&](int r, int b, float y, bool mine) {
-      put_pair(p.act, 4 * C, r, b, __float2bfloat16(gelu_tanh(y)), mine, epoch + 4);
-    });
-    copy_rows(p, sm, xs, p.act, 4 * C, epoch + 4);
-    matvec(p, sm, ring, xs, st, buf, kFc2, 4 * C, base + lay.o_b_fc2, add_to_stream(p.resid, epoch + kEpochsPerLayer));
+    // ---- next phase
+    if (which == kHead) return;
+    if (which == kFc2) {
+      ++layer;
+      if (layer == p.a.layers && p.a.logits == nullptr) return;
+      which = layer == p.a.layers ? kHead : kQkv;
+    } else {
+      ++which;
+    }
   }
-  if (p.a.logits == nullptr) return;
-  norm_rows(p.resid, epoch, lay.lnf_b >= 0);
-  matvec(p, sm, ring, xs, st, buf, kHead, C, -1, [&](int r, int b, float y, bool mine) {
-    if (mine) p.a.logits[(long long)b * p.a.vocab + r] = __bfloat162float(__float2bfloat16(y));
-  });
 }
 
 __global__ void __launch_bounds__(kThreads, 1) decode_kernel(const __grid_constant__ Params p) {
@@ -666,17 +688,19 @@ __global__ void __launch_bounds__(kThreads, 1) decode_kernel(const __grid_consta
   const DecodeLayout& lay = p.a.lay;
   const int C = p.a.C;
   bool ok = true;
-  auto opt = [](long long base, long long off) { return off < 0 ? -1ll : base + off; };
-  for (int l = 0; ok && l < p.a.layers; ++l) {
-    const long long base = lay.layer0 + l * lay.layer_stride;
-    ok = prod.norm(base + lay.o_ln1_w, opt(base, lay.o_ln1_b)) &&
-         prod.matrix(kQkv, base + lay.o_qkv, base + lay.o_b_qkv, C) &&
-         prod.matrix(kProj, base + lay.o_proj, base + lay.o_b_proj, C) &&
-         prod.norm(base + lay.o_ln2_w, opt(base, lay.o_ln2_b)) &&
-         prod.matrix(kFc, base + lay.o_fc, base + lay.o_b_fc, C) &&
-         prod.matrix(kFc2, base + lay.o_fc2, base + lay.o_b_fc2, 4 * C);
+  const int phases = 4 * p.a.layers + (p.a.logits != nullptr);
+  for (int i = 0; ok && i < phases; ++i) {  // the consumers' order; one instance of each piece of code here, too
+    const int layer = i >> 2, which = layer == p.a.layers ? kHead : i & 3;
+    const long long base = lay.layer0 + layer * lay.layer_stride;
+    if (which == kQkv || which == kFc || which == kHead) {
+      const long long w = which == kQkv ? lay.o_ln1_w : lay.o_ln2_w, b = which == kQkv ? lay.o_ln1_b : lay.o_ln2_b;
+      ok = which == kHead ? prod.norm(lay.lnf_w, lay.lnf_b) : prod.norm(base + w, b < 0 ? -1 : base + b);
+      if (!ok) break;
+    }
+    const long long w = which == kQkv ? lay.o_qkv : which == kProj ? lay.o_proj : which == kFc ? lay.o_fc : lay.o_fc2;
+    const long long b = which == kQkv ? lay.o_b_qkv : which == kProj ? lay.o_b_proj : which == kFc ? lay.o_b_fc : lay.o_b_fc2;
+    ok = prod.matrix(which, which == kHead ? lay.wte : base + w, which == kHead ? -1 : base + b, which == kFc2 ? 4 * C : C);
   }
-  if (ok && p.a.logits != nullptr) ok = prod.norm(lay.lnf_w, lay.lnf_b) && prod.matrix(kHead, lay.wte, -1, C);
   const long long issued = prod.issued;
   // the copies in flight land before this CTA's shared memory goes away; a phase that is already past
   // answers at once, and a wait that another role abandoned must not cut this one short

@@ -74,8 +74,8 @@ class TrainConfig:
     use_cuda_graph: bool = True
     overlap_wgrad: bool = True  # weight-gradient GEMMs on a second stream (fills the tails of the data-gradient chain)
     # Bitwise reproducible steps: every accumulation that normally meets in atomics runs in a fixed
-    # order instead (split-K weight gradients folded slice by slice, attention dQ one KV tile per launch,
-    # bias and embedding gradients by ordered sums). 0.86x the speed on the 124M model.
+    # order instead (split-K weight gradients folded slice by slice, attention dQ added up in KV-tile order,
+    # bias and embedding gradients by ordered sums). Slower than the default.
     deterministic: bool = False
     log_jsonl: str = ""
 
