@@ -19,7 +19,7 @@
 // the second half of their 64 columns first, so that the two rows of a quarter warp never collide.
 //
 // Between the phases the CTAs exchange activations without barriers or fences: two bf16 values travel in
-// one 8-byte store together with the number of their phase (the "epoch"), and a reader polls the data
+// one 8-byte word together with the number of their phase (the "epoch"), and a reader polls the data
 // itself until the epochs are the ones it needs. A buffer is written again one layer later, and by then
 // every CTA has handed over results that it could only compute after it had read the old contents: each of
 // the phases QKV, projection, c_fc and c_proj waits for rows of every CTA (the grid is chosen so that each
@@ -123,8 +123,11 @@ __device__ void plan(const Params& p, Smem* sm, int t) {
 }
 
 // ---- exchange ----------------------------------------------------------------------------------
+// A maximum that the L2 takes (epochs only grow, and the newer one wins): it shows earlier than a plain store
+// on a line that other SMs are polling (one token: 124M model 230 -> 206 us, 1.5B for four sequences 1.65 ->
+// 1.50 ms).
 __device__ __forceinline__ void put(uint64_t* p, uint32_t value, uint32_t epoch) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((uint64_t)epoch << 32 | value) : "memory");
+  asm volatile("red.relaxed.gpu.global.max.u64 [%0], %1;" ::"l"(p), "l"((uint64_t)epoch << 32 | value) : "memory");
 }
 struct Units2 {
   uint64_t a, b;
@@ -178,11 +181,6 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// One instance of the bounded wait for all its places.
-__device__ __noinline__ bool wait_for(Smem* sm, uint64_t* bar, uint32_t phase, int* status, int code) {
-  return mbar_wait_bounded(bar, phase, &sm->abort_flag, status, code);
-}
-
 // ---- producer (a warp) --------------------------------------------------------------------------
 struct Ring {
   int slot = 0;
@@ -202,7 +200,7 @@ struct Producer {
 
   // lane 0 has the slot's transaction count armed on return
   __device__ __noinline__ bool open(uint32_t bytes) {
-    const bool ok = wait_for(sm, &sm->empty[st.slot], st.phase ^ 1, p.a.status, kTimeoutEmpty);
+    const bool ok = mbar_wait_bounded(&sm->empty[st.slot], st.phase ^ 1, &sm->abort_flag, p.a.status, kTimeoutEmpty);
     if (!__all_sync(0xffffffffu, ok)) return false;
     if ((threadIdx.x & 31) == 0) mbar_arrive_expect_tx(&sm->full[st.slot], bytes);
     __syncwarp();
@@ -270,7 +268,7 @@ __device__ __forceinline__ void matvec(const Params& p, Smem* sm, const uint8_t*
     float acc[4][4] = {}, add = 0.f;  // four chains: a step's products do not wait for each other
     for (int k = 0; k < K; k += own.cols) {
       const int n = min(own.cols, K - k);
-      wait_for(sm, &sm->full[st.slot], st.phase, p.a.status, kTimeoutFull);
+      mbar_wait_bounded(&sm->full[st.slot], st.phase, &sm->abort_flag, p.a.status, kTimeoutFull);
       const uint8_t* slot = ring + (size_t)st.slot * (p.slot_bytes + kBiasBytes);
       if (k == 0 && bias >= 0 && mine)
         add = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(slot + p.slot_bytes)[((bias + r) & 7) + in_tile]);
@@ -396,7 +394,7 @@ __device__ __forceinline__ void layer_norm_rows(const Params& p, Smem* sm, const
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
     const float rstd = rsqrtf(sq / C + 1e-5f);
-    wait_for(sm, &sm->full[st.slot], st.phase, p.a.status, kTimeoutFull);
+    mbar_wait_bounded(&sm->full[st.slot], st.phase, &sm->abort_flag, p.a.status, kTimeoutFull);
     const uint8_t* norm = ring + (size_t)st.slot * (p.slot_bytes + kBiasBytes);
 #pragma unroll 1
     for (int c = lane * 8; c < C; c += 256) {
@@ -581,7 +579,8 @@ __device__ __forceinline__ void fold_attention(const Params& p, Smem* sm, uint8_
 
 // One loop over the phases of all layers with a single instance of each piece of code: laid out phase by
 // phase the kernel was 170 KB of code (65 KB now) and every phase began with instruction-cache misses (one
-// token of the 124M model 330 us, 248 so; of the 1.5B model for four sequences 2.4 and 1.7 ms).
+// token of the 124M model 330 us, 230 so; of the 1.5B model for four sequences 2.4 and 1.65 ms). The bounded
+// waits are inlined all the same: out of line each cost some 500 cycles.
 __device__ __forceinline__ void consume(const Params& p, Smem* sm, const uint8_t* ring, uint8_t* xs) {
   const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(p.a.weights);
   const DecodeLayout& lay = p.a.lay;

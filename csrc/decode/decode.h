@@ -21,7 +21,7 @@ struct DecodeArgs {
   long long token_stride;
   float* logits;            // fp32 [batch][vocab], rounded to bf16 like the module's; null: no head
   void* scratch;            // decode_scratch_bytes(), zeroed once before the first step
-  unsigned int epoch_base;  // 1 in the first step on this scratch, then decode_epochs() more in each
+  unsigned int epoch_base;  // 1 in the first step on this scratch, then decode_epochs() more in each (never less)
   int batch, C, heads, layers, vocab, pos, max_len;
   int* status;
 };

@@ -16,7 +16,7 @@ from . import _lib, gemm as G, native as N
 MAX_BATCH = 8            # sequences of one decode launch (the n of its tensor-core instruction)
 MAX_SEQUENCES = 32       # sequences of a session, in groups of MAX_BATCH
 # A prompt of up to this many tokens goes through the decode kernel one by one: on a B200 one token of
-# the 124M model takes about 0.1 ms there, while the batched pass is bound by its ~100 launches.
+# the 124M model takes about 0.2 ms there, while the batched pass is bound by its ~100 launches.
 STEPWISE_PROMPT = 6
 
 _sigs = {
@@ -187,7 +187,7 @@ class DecodeSession:
             _call("z2h_decode_step", self.numbers, _lib.ptr(self.w), _lib.ptr(g["kv"]),
                   ctypes.c_void_p(tokens.data_ptr() + 8 * b0 * stride), stride, logits, _lib.ptr(g["scratch"]),
                   g["base"], g["n"], self.C, self.H, self.L, self.V, pos, self.max_len, status, stream)
-            g["base"] = (g["base"] + g["epochs"]) & 0xFFFFFFFF
+            g["base"] += g["epochs"]  # 32 bits hold some 10^7 steps of the largest model
         return self.logits
 
     def prefill(self, tokens: torch.Tensor) -> None:
