@@ -15,9 +15,11 @@ from . import _lib, gemm as G, native as N
 
 MAX_BATCH = 8            # sequences of one decode launch (the n of its tensor-core instruction)
 MAX_SEQUENCES = 32       # sequences of a session, in groups of MAX_BATCH
-# A prompt of up to this many tokens goes through the decode kernel one by one: on a B200 one token of
-# the 124M model takes about 0.2 ms there, while the batched pass is bound by its ~100 launches.
-STEPWISE_PROMPT = 6
+# A prompt of up to this many tokens (before its last one) goes through the decode kernel one by one, a longer
+# one through the batched pass, which is bound by its launches. Stepwise / batched, ms: 124M, one sequence, 4
+# tokens 0.74 / 1.09, 6 tokens 1.11 / 1.08; eight sequences, 4 tokens 1.02 / 1.08; 1.5B, 4 tokens 4.4 / 5.0,
+# 6 tokens 6.6 / 5.0.
+STEPWISE_PROMPT = 4
 
 _sigs = {
     "z2h_decode_scratch_bytes": ([ctypes.c_int] * 3, ctypes.c_longlong),
