@@ -9,12 +9,13 @@ int ce_fwd_bwd(void* logits, const void* targets, int idx_is_64, float* losses, 
                int V_pad, long long ld, float grad_scale, int write_grad, int ignore_index,
                cudaStream_t stream);
 // The pair behind autograd: the forward leaves the logits alone (any pitch and 2-byte alignment; rows of
-// up to 57,300 columns) and writes losses, log-sum-exps and, unless null, a copy of the logits with zeros
-// up to the next multiple of 8 columns; the backward turns that copy (same pitch) into
+// up to 57,300 columns) and writes losses, every row's maximum and logarithm of the sum of exp(x - maximum)
+// (`stats`, two floats a row) and, unless null, a copy of the logits with zeros up to the next multiple of 8
+// columns; the backward turns that copy (same pitch) into
 // (softmax - onehot) * scale * *upstream.
-int ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* lse,
+int ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* stats,
                 void* copy, long long ld_copy, int M, int V, int V_real, int ignore_index, cudaStream_t stream);
-int ce_bwd(const void* x, const void* targets, int idx_is_64, const float* lse, const float* upstream, float scale,
+int ce_bwd(const void* x, const void* targets, int idx_is_64, const float* stats, const float* upstream, float scale,
            void* grad, long long ld, int M, int V, int V_real, int ignore_index, cudaStream_t stream);
 // dst (tight bf16 rows of N) = src (rows of pitch ld)
 int compact_rows(const void* src, long long ld, void* dst, int M, int N, cudaStream_t stream);

@@ -278,7 +278,7 @@ struct RowWindow {
 template <typename IdxT, bool SHIFT>
 __global__ void __launch_bounds__(kRowThreads)
 ce_fwd_save_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, const IdxT* __restrict__ targets,
-                   float* __restrict__ losses, float* __restrict__ lse_out, __nv_bfloat16* __restrict__ copy,
+                   float* __restrict__ losses, float2* __restrict__ stats, __nv_bfloat16* __restrict__ copy,
                    long long ld_copy, int V, int V_real, int ignore_index, int* status) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ float sh[32];
@@ -326,7 +326,6 @@ ce_fwd_save_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, const
     }
   }
   m = cta_reduce<true>(m, sh);
-  const float m2 = m * kLog2e;
   float s = 0.f;
   for (int v = threadIdx.x; v < nvec; v += kRowThreads) {
     const uint4 u = win.vec<SHIFT>(v);
@@ -335,30 +334,31 @@ ce_fwd_save_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, const
     for (int j = 0; j < 4; ++j) {
       const float2 f = unpack_bf16x2(w[j]);
       const int c = v * 8 + 2 * j;
-      const float e0 = ex2_fast(fmaf(f.x, kLog2e, -m2)), e1 = ex2_fast(fmaf(f.y, kLog2e, -m2));
+      // the maximum is subtracted before the scaling: m * log2(e) overflows for a row of the type's lowest value
+      const float e0 = ex2_fast((f.x - m) * kLog2e), e1 = ex2_fast((f.y - m) * kLog2e);
       s += (c < V_real ? e0 : 0.f) + (c + 1 < V_real ? e1 : 0.f);
     }
   }
   s = cta_reduce<false>(s, sh);
   if (threadIdx.x == 0) {
-    const float lse = m + logf(s);
-    lse_out[row] = lse;
-    losses[row] = ignored ? 0.f : lse - __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(smem)[win.shift + tgt]);
+    const float log_s = logf(s);
+    stats[row] = make_float2(m, log_s);  // apart: a large maximum would swallow the logarithm
+    losses[row] = ignored ? 0.f : log_s + (m - __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(smem)[win.shift + tgt]));
     if (!SHIFT && copy != nullptr) tma_store_wait_read<0>();  // shared memory stays until the copy has read it
   }
 }
 
-// grad = (exp(x - lse) - onehot) * scale * *upstream: one read, one write, rounded once. Two rows in
-// flight per SM hide the loads; a thread keeps four vectors in flight.
+// grad = (exp(x - max - log sum) - onehot) * scale * *upstream: one read, one write, rounded once. Two rows
+// in flight per SM hide the loads; a thread keeps four vectors in flight.
 template <typename IdxT>
 __global__ void __launch_bounds__(kThreads)
-ce_bwd_kernel(const __nv_bfloat16* __restrict__ x, const IdxT* __restrict__ targets, const float* __restrict__ lse,
+ce_bwd_kernel(const __nv_bfloat16* __restrict__ x, const IdxT* __restrict__ targets, const float2* __restrict__ stats,
               const float* __restrict__ upstream, float scale, __nv_bfloat16* __restrict__ grad, long long ld, int V,
               int V_real, int ignore_index) {
   const int row = blockIdx.x, nvec = (V + 7) / 8;
   const long long tgt = (long long)targets[row];
   const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V_real;
-  const float g = ignored ? 0.f : *upstream * scale, l2 = lse[row] * kLog2e;
+  const float g = ignored ? 0.f : *upstream * scale, m = stats[row].x, l2 = stats[row].y * kLog2e;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (long long)row * ld);
   uint4* gr = reinterpret_cast<uint4*>(grad + (long long)row * ld);
 #pragma unroll 4
@@ -369,7 +369,7 @@ ce_bwd_kernel(const __nv_bfloat16* __restrict__ x, const IdxT* __restrict__ targ
     for (int j = 0; j < 4; ++j) {
       const float2 f = unpack_bf16x2(w[j]);
       const int c = v * 8 + 2 * j;
-      float a = ex2_fast(fmaf(f.x, kLog2e, -l2)), b = ex2_fast(fmaf(f.y, kLog2e, -l2));
+      float a = ex2_fast(fmaf(f.x - m, kLog2e, -l2)), b = ex2_fast(fmaf(f.y - m, kLog2e, -l2));
       if (c == tgt) a -= 1.f;
       if (c + 1 == tgt) b -= 1.f;
       w[j] = pack_bf16x2(c < V_real && !ignored ? a * g : 0.f, c + 1 < V_real && !ignored ? b * g : 0.f);
@@ -448,7 +448,7 @@ int ce_fwd_bwd(void* logits, const void* targets, int idx_is_64, float* losses, 
 }
 
 template <typename IdxT>
-static int ce_fwd_save_t(const void* logits, long long ld, const void* targets, float* losses, float* lse, void* copy,
+static int ce_fwd_save_t(const void* logits, long long ld, const void* targets, float* losses, float2* stats, void* copy,
                          long long ld_copy, int M, int V, int V_real, int ignore_index, cudaStream_t stream) {
   const bool shift = (ld % 8) != 0 || (reinterpret_cast<uintptr_t>(logits) & 15) || V % 8 != 0;
   const size_t smem = (size_t)((V + 7 + 7) / 8 * 8 + 8) * 2;  // the row, up to 7 columns before it, a word after
@@ -459,31 +459,34 @@ static int ce_fwd_save_t(const void* logits, long long ld, const void* targets, 
     cudaFuncSetAttribute(ce_fwd_save_kernel<IdxT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowMaxBytes);
   }
   auto kern = shift ? ce_fwd_save_kernel<IdxT, true> : ce_fwd_save_kernel<IdxT, false>;
-  kern<<<M, kRowThreads, smem, stream>>>((const __nv_bfloat16*)logits, ld, (const IdxT*)targets, losses, lse,
+  kern<<<M, kRowThreads, smem, stream>>>((const __nv_bfloat16*)logits, ld, (const IdxT*)targets, losses, stats,
                                          (__nv_bfloat16*)copy, ld_copy, V, V_real, ignore_index, nullptr);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
-int ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* lse,
+int ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* stats,
                 void* copy, long long ld_copy, int M, int V, int V_real, int ignore_index, cudaStream_t stream) {
   if (M <= 0) return 0;
   if (V < 1 || V_real < 1 || V_real > V || ld < V || (reinterpret_cast<uintptr_t>(logits) & 1)) return 1;
   if (copy != nullptr && (ld_copy % 8 || ld_copy < (V + 7) / 8 * 8 || (reinterpret_cast<uintptr_t>(copy) & 15))) return 1;
-  return idx_is_64 ? ce_fwd_save_t<long long>(logits, ld, targets, losses, lse, copy, ld_copy, M, V, V_real, ignore_index, stream)
-                   : ce_fwd_save_t<int>(logits, ld, targets, losses, lse, copy, ld_copy, M, V, V_real, ignore_index, stream);
+  if (reinterpret_cast<uintptr_t>(stats) & 7) return 1;
+  auto f = idx_is_64 ? ce_fwd_save_t<long long> : ce_fwd_save_t<int>;
+  return f(logits, ld, targets, losses, reinterpret_cast<float2*>(stats), copy, ld_copy, M, V, V_real, ignore_index,
+           stream);
 }
 
-int ce_bwd(const void* x, const void* targets, int idx_is_64, const float* lse, const float* upstream, float scale,
+int ce_bwd(const void* x, const void* targets, int idx_is_64, const float* stats, const float* upstream, float scale,
            void* grad, long long ld, int M, int V, int V_real, int ignore_index, cudaStream_t stream) {
   if (M <= 0) return 0;
   if (V < 1 || V_real < 1 || V_real > V || ld % 8 || ld < (V + 7) / 8 * 8 ||
-      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(grad)) & 15))
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(grad)) & 15) || (reinterpret_cast<uintptr_t>(stats) & 7))
     return 1;
+  const float2* st = reinterpret_cast<const float2*>(stats);
   if (idx_is_64)
-    ce_bwd_kernel<long long><<<M, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (const long long*)targets, lse, upstream,
+    ce_bwd_kernel<long long><<<M, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (const long long*)targets, st, upstream,
                                                          scale, (__nv_bfloat16*)grad, ld, V, V_real, ignore_index);
   else
-    ce_bwd_kernel<int><<<M, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (const int*)targets, lse, upstream, scale,
+    ce_bwd_kernel<int><<<M, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (const int*)targets, st, upstream, scale,
                                                    (__nv_bfloat16*)grad, ld, V, V_real, ignore_index);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
@@ -509,14 +512,14 @@ int z2h_ce_fwd_bwd(void* logits, const void* targets, int idx_is_64, float* loss
   return z2h::ce_fwd_bwd(logits, targets, idx_is_64, losses, M, V_real, V_pad, ld, grad_scale,
                          write_grad, ignore_index, (cudaStream_t)stream);
 }
-int z2h_ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* lse,
+int z2h_ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* stats,
                     void* copy, long long ld_copy, int M, int V, int V_real, int ignore_index, void* stream) {
-  return z2h::ce_fwd_save(logits, ld, targets, idx_is_64, losses, lse, copy, ld_copy, M, V, V_real, ignore_index,
+  return z2h::ce_fwd_save(logits, ld, targets, idx_is_64, losses, stats, copy, ld_copy, M, V, V_real, ignore_index,
                           (cudaStream_t)stream);
 }
-int z2h_ce_bwd(const void* x, const void* targets, int idx_is_64, const float* lse, const float* upstream, float scale,
+int z2h_ce_bwd(const void* x, const void* targets, int idx_is_64, const float* stats, const float* upstream, float scale,
                void* grad, long long ld, int M, int V, int V_real, int ignore_index, void* stream) {
-  return z2h::ce_bwd(x, targets, idx_is_64, lse, upstream, scale, grad, ld, M, V, V_real, ignore_index,
+  return z2h::ce_bwd(x, targets, idx_is_64, stats, upstream, scale, grad, ld, M, V, V_real, ignore_index,
                      (cudaStream_t)stream);
 }
 int z2h_compact_rows(const void* src, long long ld, void* dst, int M, int N, void* stream) {

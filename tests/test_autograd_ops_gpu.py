@@ -66,6 +66,29 @@ def test_cross_entropy_other_forms_keep_their_results():
     assert float(Z.cross_entropy(lowest, torch.tensor([5, 5], device="cuda"))) == 0.0
 
 
+# rows of one value, so large that its multiple by log2(e) leaves fp32: the loss is log V whatever the value is;
+# widths of both routes, and one where the rows start anywhere
+@pytest.mark.parametrize("V", (33, 40, 50257))
+def test_cross_entropy_of_the_largest_values(V):
+    from zero_to_hero_b200.ops import functional as Z
+
+    top = torch.finfo(torch.bfloat16).max
+    for value in (-top, top, -1e5, 1e5):
+        x = torch.full((3, V), value).bfloat16().cuda()
+        x[1, 5:] = 0.0  # beside another row: one class, or all but five, take everything
+        t = torch.tensor([1, 2, V - 1], device="cuda")
+        ref = x.double().requires_grad_()
+        F.cross_entropy(ref[[0, 2]], t[[0, 2]]).backward()
+        x.requires_grad_()
+        loss = Z.cross_entropy(x, t)
+        rows = torch.stack([Z.cross_entropy(x[i:i + 1].detach(), t[i:i + 1]) for i in range(3)])
+        want = F.cross_entropy(x.detach().float(), t, reduction="none")
+        assert torch.allclose(rows, want, rtol=1e-6, atol=1e-6), (value, rows, want)
+        loss.backward()
+        assert x.grad.isfinite().all()
+        assert _rel(x.grad[[0, 2]] * 1.5, ref.grad[[0, 2]]) < BF16
+
+
 @pytest.mark.parametrize("M,K,N,bias", [(1, 8, 1, True), (300, 384, 65, True), (130, 64, 127, False),
                                         (2048, 64, 257, True), (33, 768, 50257, False)])
 def test_linear_of_any_width(M, K, N, bias):

@@ -386,14 +386,14 @@ class _CrossEntropySaved(torch.autograd.Function):
         M, V = logits.shape
         targets = targets.contiguous()
         losses = torch.empty(M, device=logits.device, dtype=torch.float32)
-        lse = torch.empty_like(losses)
+        stats = torch.empty(M, 2, device=logits.device, dtype=torch.float32)
         copy = None
         if ctx.needs_input_grad[0]:
             copy = torch.empty(M, (V + 7) // 8 * 8, device=logits.device, dtype=torch.bfloat16)
-        N.ce_fwd_save(logits, targets, losses, lse, copy, v_real)
+        N.ce_fwd_save(logits, targets, losses, stats, copy, v_real)
         count = (targets != -100).sum().float() if skip_ignored else None
         if copy is not None:
-            ctx.save_for_backward(copy, targets, lse, count)
+            ctx.save_for_backward(copy, targets, stats, count)
             ctx.meta = (M, V, v_real)
             # a second derivative goes through the caller's logits themselves
             ctx.logits, ctx.version = (logits, logits._version) if skip_ignored else (None, 0)
@@ -401,7 +401,7 @@ class _CrossEntropySaved(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        copy, targets, lse, count = ctx.saved_tensors
+        copy, targets, stats, count = ctx.saved_tensors
         M, V, v_real = ctx.meta
         skipping = count is not None
         if torch.is_grad_enabled() and (g.requires_grad or skipping):  # a graph of this backward is wanted
@@ -409,12 +409,12 @@ class _CrossEntropySaved(torch.autograd.Function):
             x = x[:, :v_real].float()
             valid = ((targets >= 0) & (targets < v_real)).float()
             hit = (targets[:, None] == torch.arange(v_real, device=x.device)).float()
-            p = x.softmax(1) if skipping else torch.exp(x - lse[:, None])
+            p = x.softmax(1) if skipping else torch.exp(x - stats[:, :1] - stats[:, 1:])
             grad = F.pad((p - hit) * valid[:, None], (0, V - v_real))
             return (grad * (g / count if skipping else g / M)).bfloat16(), None, None, None
         grad = torch.empty_like(copy)
         up = g / count if skipping else g
-        N.ce_bwd(copy, targets, lse, up.reshape(1), 1.0 if skipping else 1.0 / M, grad, V, v_real)
+        N.ce_bwd(copy, targets, stats, up.reshape(1), 1.0 if skipping else 1.0 / M, grad, V, v_real)
         return grad[:, :V], None, None, None
 
 
