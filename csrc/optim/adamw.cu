@@ -204,7 +204,7 @@ long long colsum_scratch_elems(int M, int N) {
 
 int colsum_bf16_ordered(const void* dy, int M, int N, long long ld, float* db, int accumulate, int ordered,
                         float* scratch, cudaStream_t stream) {
-  if (N % 8 != 0 || ld % 8 != 0) return 1;
+  if (N % 8 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(dy) & 15)) return 1;  // 16-byte loads
   if (!accumulate) cudaMemsetAsync(db, 0, sizeof(float) * N, stream);
   const bool two_stage = ordered && scratch != nullptr;
   int slabs = (ordered && !two_stage) ? 1 : (M + 127) / 128;

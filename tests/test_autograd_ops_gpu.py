@@ -111,6 +111,31 @@ def test_linear_of_any_width(M, K, N, bias):
     assert not bias or _rel(b.grad, rb.grad) < BF16
 
 
+# an upstream gradient that starts between two 16-byte boundaries, for every epilogue of the forward and with
+# the bias alone wanted
+@pytest.mark.parametrize("act,residual,frozen", [("gelu_tanh", False, False), (None, False, False), (None, True, False),
+                                                 (None, False, True)])
+def test_linear_takes_a_gradient_of_any_alignment(act, residual, frozen):
+    from zero_to_hero_b200.ops import functional as Z, native
+
+    g = torch.Generator().manual_seed(3)
+    x, w, b, r = (torch.randn(*s, generator=g).bfloat16().cuda() for s in ((24, 64), (72, 64), (72,), (24, 72)))
+    for t in (x, w):
+        t.requires_grad_(not frozen)
+    b.requires_grad_()
+    up = torch.randn(24 * 72 + 1, generator=g).bfloat16().cuda()[1:].view(24, 72)
+    assert up.data_ptr() % 16
+    Z.linear(x, w, b, act, r if residual else None).backward(up)
+    got = [t.grad for t in (x, w, b)]
+    for t in (x, w, b):
+        t.grad = None
+    Z.linear(x, w, b, act, r if residual else None).backward(up.clone())
+    assert all((p is None and t.grad is None) or torch.equal(p, t.grad) for p, t in zip(got, (x, w, b)))
+    assert frozen == (x.grad is None) and b.grad is not None
+    with pytest.raises(RuntimeError):  # refused by the host, nothing is launched
+        native.colsum_bf16(up, torch.zeros(72, device="cuda"))
+
+
 @pytest.mark.parametrize("M,N", [(1, 8), (33, 264), (1000, 256), (4099, 3072)])
 def test_gelu_backward(M, N):
     from zero_to_hero_b200.ops import native

@@ -68,6 +68,12 @@ def _gemm_ok(*dims: int) -> bool:
     return all(d % 8 == 0 for d in dims)
 
 
+def _tight(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and on the 16-byte boundary the tensor maps and the vector loads need."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 # --------------------------------------------------------------------------------------------
 # linear
 # --------------------------------------------------------------------------------------------
@@ -112,7 +118,7 @@ class _Linear(torch.autograd.Function):
         M, K = x2.shape
         Nout = w16.shape[0]
         dy2 = dy.reshape(M, Nout)
-        dy2 = (dy2 if dy2.dtype == torch.bfloat16 else dy2.bfloat16()).contiguous()
+        dy2 = _tight(dy2 if dy2.dtype == torch.bfloat16 else dy2.bfloat16())
         dres = dy2.reshape(dy.shape).to(ctx.res_dtype) if ctx.has_res else None
         dx = dw = db32 = None
         want_db = ctx.has_bias and ctx.needs_input_grad[2]
@@ -140,12 +146,6 @@ class _Linear(torch.autograd.Function):
 def _transformed() -> bool:
     """Inside a function transform (vmap, torch.func.grad) or forward-mode differentiation."""
     return torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0
-
-
-def _tight(t: torch.Tensor) -> torch.Tensor:
-    """Contiguous and on the 16-byte boundary the tensor maps need."""
-    t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 class _LinearAnyWidth(torch.autograd.Function):
