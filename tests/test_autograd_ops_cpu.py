@@ -1,0 +1,26 @@
+"""Which calls of the autograd ops take the kernels for unpadded widths (rules only, on the CPU)."""
+import torch
+
+from zero_to_hero_b200.ops import functional as Z
+
+
+def test_odd_widths_take_the_kernels_only_for_what_they_compute():
+    def ok(x, w, b=None):
+        return Z._any_width_ok(x, w, b)
+
+    x, w = torch.zeros(2, 3, 16), torch.zeros(7, 16)
+    assert ok(x, w) and ok(x, w, torch.zeros(7)) and ok(x[0, 0], w) and ok(x.bfloat16(), w.double())
+    for b in (torch.zeros(1), torch.zeros(()), torch.zeros(1, 7), torch.zeros(6)):  # broadcast or refused by F.linear
+        assert not ok(x, w, b)
+    assert not ok(x, torch.zeros(7, 8)) and not ok(x, torch.zeros(16)) and not ok(x[:0], w) and not ok(x, w[:0])
+    elsewhere = torch.zeros(7, 16, device="meta")
+    assert not ok(x, elsewhere) and not ok(x, w, elsewhere[:, 0])
+    with torch.autocast("cpu", dtype=torch.bfloat16):
+        assert ok(x, w)
+    with torch.autocast("cpu", dtype=torch.float16):
+        assert not ok(x, w)
+    torch.use_deterministic_algorithms(True)
+    try:
+        assert not ok(x, w)
+    finally:
+        torch.use_deterministic_algorithms(False)

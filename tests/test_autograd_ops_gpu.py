@@ -151,3 +151,14 @@ def test_gelu_backward(M, N):
     ok = torch.isfinite(ref.grad)  # fp64's own x^3 stays finite where fp32's overflows: both end at 0 or dy
     assert _rel(dx[ok], ref.grad[ok]) < BF16 and torch.isfinite(dx).all()
     assert torch.allclose(db.double(), 1 + dx.double().sum(0), rtol=1e-4, atol=1e-4 * M ** 0.5)
+
+
+def test_odd_widths_that_the_kernels_do_not_compute_keep_the_library():
+    from zero_to_hero_b200.ops import functional as Z
+
+    x, w = torch.randn(5, 64).cuda(), torch.randn(7, 64).cuda()
+    for b in (torch.full((1,), 2.0).cuda(), torch.full((1, 7), 2.0).cuda()):  # broadcast
+        assert torch.equal(Z.linear(x, w, b), F.linear(x.bfloat16(), w.bfloat16(), b.bfloat16()))
+    for bad in ((x, w[:, :32]), (x, w.cpu()), (x, w, torch.zeros(6).cuda()), (x, w, torch.zeros(7))):
+        with pytest.raises(RuntimeError):  # F.linear's own refusal, on the host
+            Z.linear(*bad)

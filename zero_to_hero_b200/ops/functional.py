@@ -148,6 +148,20 @@ def _transformed() -> bool:
     return torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0
 
 
+def _any_width_ok(x, w, b) -> bool:
+    """Whether `_LinearAnyWidth` computes what F.linear over bf16 casts does here. Anything that F.linear refuses,
+    broadcasts or computes in another type or order goes to it: the kernels take plain addresses."""
+    if w.dim() != 2 or x.dim() < 1 or w.shape[1] != x.shape[-1] or x.numel() == 0 or w.numel() == 0:
+        return False
+    if b is not None and b.shape != w.shape[:1]:
+        return False
+    if any(t.device != x.device for t in (w, b) if t is not None):
+        return False
+    if torch.is_autocast_enabled(x.device.type) and torch.get_autocast_dtype(x.device.type) != torch.bfloat16:
+        return False
+    return not torch.are_deterministic_algorithms_enabled()  # the weight gradient may add with atomics
+
+
 class _LinearAnyWidth(torch.autograd.Function):
     """y = x @ w.T + b over bf16 tensors for output widths that are no multiple of 8 (an unpadded
     vocabulary): the tensor cores work on a 16-byte pitch, the caller gets tight rows."""
@@ -202,8 +216,7 @@ def linear(x, w, b=None, act: str | None = None, residual=None):
     K, Nout = x.shape[-1], w.shape[0]
     if _native(x) and _gemm_ok(K, Nout):
         return _Linear.apply(x, w, b, act, residual)
-    if _native(x) and _gemm_ok(K) and act is None and residual is None and w.dim() == 2 and x.numel() > 0 and \
-            w.numel() > 0 and not _transformed():
+    if _native(x) and _gemm_ok(K) and act is None and residual is None and not _transformed() and _any_width_ok(x, w, b):
         return _LinearAnyWidth.apply(x.bfloat16(), w.bfloat16(), None if b is None else b.bfloat16())
     if _native(x):
         FALLBACK_COUNTS["linear"] += 1
