@@ -24,3 +24,28 @@ def test_odd_widths_take_the_kernels_only_for_what_they_compute():
         assert not ok(x, w)
     finally:
         torch.use_deterministic_algorithms(False)
+
+
+def test_traces_and_transforms_are_seen():
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    seen = []
+
+    def look(x):
+        seen.append(Z._transformed())
+        return x * 2.0
+
+    x = torch.ones(3)
+    look(x)
+    assert seen == [False]
+    torch.func.vmap(look)(x)
+    torch.func.jvp(look, (x,), (x,))
+    torch.func.grad(lambda v: look(v).sum())(x)
+    torch.jit.trace(look, (x,), check_trace=False)
+    make_fx(look)(x)
+    with FakeTensorMode():
+        look(torch.ones(3))
+    assert len(seen) == 7 and all(seen[1:])
+    look(x)
+    assert not seen[-1]

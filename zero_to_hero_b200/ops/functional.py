@@ -144,7 +144,11 @@ class _Linear(torch.autograd.Function):
 
 
 def _transformed() -> bool:
-    """Inside a function transform (vmap, torch.func.grad) or forward-mode differentiation."""
+    """Inside a function transform (vmap, torch.func.grad), forward-mode differentiation, a trace (compile, jit,
+    make_fx) or a dispatch mode (fake tensors): a launch through plain addresses would be missing from what is
+    transformed or recorded."""
+    if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0:
+        return True
     return torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0
 
 
