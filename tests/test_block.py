@@ -47,7 +47,11 @@ def test_only_plain_blocks_are_fused():
     assert not char(lambda b: setattr(b.ff.ff, "1", nn.GELU()))
     from zero_to_hero_b200.ops import block as FB
     assert not FB.usable(torch.zeros(1, 2, 128, dtype=torch.bfloat16), 2, [torch.zeros(128)])  # not on a GPU
-    assert not FB.shaped([torch.zeros(3), None], ((3,), (3, 3))) and FB.shaped([torch.zeros(3), None], ((3,), (3,)))
+    whole = [torch.zeros(3)] * 12
+    shapes = ((3,),) * 12
+    assert FB.shaped(whole, shapes) and not FB.shaped(whole, shapes[:11]) and not FB.shaped(whole, shapes[:11] + ((3, 3),))
+    for i in range(12):  # in the order of the node's parameters: only biases may be absent
+        assert FB.shaped([None if j == i else t for j, t in enumerate(whole)], shapes) == (i in (1, 2, 4, 6, 8, 10))
 
 
 def _grads(model, X, Y):

@@ -18,8 +18,7 @@ from . import gemm as G, native as N
 from .functional import pick_split_k
 
 _ORDER = ("ln1_w", "ln1_b", "b_qkv", "w_proj", "b_proj", "ln2_w", "ln2_b", "w_fc", "b_fc", "w_fc2", "b_fc2")
-
-
+_BIASES = ("ln1_b", "b_qkv", "b_proj", "ln2_b", "b_fc", "b_fc2")
 _SHAPES = {"w_proj": (1, 1), "w_fc": (4, 1), "w_fc2": (1, 4)}  # in units of C
 
 
@@ -37,9 +36,10 @@ def usable(x: torch.Tensor, num_heads: int, params) -> bool:
 
 
 def shaped(params, shapes) -> bool:
-    """The parameters have these shapes (biases may be absent)."""
+    """The parameters, those of `_ORDER` and the row blocks of the QKV weight, have these shapes; biases may be
+    absent, and nothing else (the kernels would read a weight that is not there at address 0)."""
     return len(params) == len(shapes) and all(p is None or tuple(p.shape) == s for p, s in zip(params, shapes)) and \
-        all(p is not None for p, s in zip(params, shapes) if s is not None and len(s) == 2)
+        all(p is not None or name in _BIASES for p, name in zip(params, _ORDER + ("w_qkv",) * (len(params) - len(_ORDER))))
 
 
 def plain_modules(pairs) -> bool:
