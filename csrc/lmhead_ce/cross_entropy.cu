@@ -275,11 +275,17 @@ struct RowWindow {
   }
 };
 
+// strict: a label that names neither a class nor ignore_index is an error, which shows as a NaN in the loss and
+// the gradient and in the status word; otherwise such a row counts as ignored.
+__device__ __forceinline__ bool bad_label(long long tgt, int V_real, int ignore_index, int strict) {
+  return strict && tgt != ignore_index && (tgt < 0 || tgt >= V_real);
+}
+
 template <typename IdxT, bool SHIFT>
 __global__ void __launch_bounds__(kRowThreads)
 ce_fwd_save_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, const IdxT* __restrict__ targets,
                    float* __restrict__ losses, float2* __restrict__ stats, __nv_bfloat16* __restrict__ copy,
-                   long long ld_copy, int V, int V_real, int ignore_index, int* status) {
+                   long long ld_copy, int V, int V_real, int ignore_index, int strict, int* status) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ float sh[32];
   __shared__ __align__(8) uint64_t bar;
@@ -343,7 +349,13 @@ ce_fwd_save_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, const
   if (threadIdx.x == 0) {
     const float log_s = logf(s);
     stats[row] = make_float2(m, log_s);  // apart: a large maximum would swallow the logarithm
-    losses[row] = ignored ? 0.f : log_s + (m - __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(smem)[win.shift + tgt]));
+    float loss = 0.f;
+    if (!ignored) loss = log_s + (m - __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(smem)[win.shift + tgt]));
+    if (bad_label(tgt, V_real, ignore_index, strict)) {
+      loss = NAN;
+      if (status != nullptr) atomicCAS(status, 0, (int)kBadArgument);
+    }
+    losses[row] = loss;
     if (!SHIFT && copy != nullptr) tma_store_wait_read<0>();  // shared memory stays until the copy has read it
   }
 }
@@ -354,11 +366,12 @@ template <typename IdxT>
 __global__ void __launch_bounds__(kThreads)
 ce_bwd_kernel(const __nv_bfloat16* __restrict__ x, const IdxT* __restrict__ targets, const float2* __restrict__ stats,
               const float* __restrict__ upstream, float scale, __nv_bfloat16* __restrict__ grad, long long ld, int V,
-              int V_real, int ignore_index) {
+              int V_real, int ignore_index, int strict) {
   const int row = blockIdx.x, nvec = (V + 7) / 8;
   const long long tgt = (long long)targets[row];
-  const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V_real;
-  const float g = ignored ? 0.f : *upstream * scale, m = stats[row].x, l2 = stats[row].y * kLog2e;
+  const bool bad = bad_label(tgt, V_real, ignore_index, strict);
+  const bool ignored = !bad && ((tgt == ignore_index) || tgt < 0 || tgt >= V_real);
+  const float g = bad ? NAN : ignored ? 0.f : *upstream * scale, m = stats[row].x, l2 = stats[row].y * kLog2e;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (long long)row * ld);
   uint4* gr = reinterpret_cast<uint4*>(grad + (long long)row * ld);
 #pragma unroll 4
@@ -449,7 +462,8 @@ int ce_fwd_bwd(void* logits, const void* targets, int idx_is_64, float* losses, 
 
 template <typename IdxT>
 static int ce_fwd_save_t(const void* logits, long long ld, const void* targets, float* losses, float2* stats, void* copy,
-                         long long ld_copy, int M, int V, int V_real, int ignore_index, cudaStream_t stream) {
+                         long long ld_copy, int M, int V, int V_real, int ignore_index, int strict, int* status,
+                         cudaStream_t stream) {
   const bool shift = (ld % 8) != 0 || (reinterpret_cast<uintptr_t>(logits) & 15) || V % 8 != 0;
   const size_t smem = (size_t)((V + 7 + 7) / 8 * 8 + 8) * 2;  // the row, up to 7 columns before it, a word after
   if (smem > (size_t)kRowMaxBytes) return 1;
@@ -460,23 +474,24 @@ static int ce_fwd_save_t(const void* logits, long long ld, const void* targets, 
   }
   auto kern = shift ? ce_fwd_save_kernel<IdxT, true> : ce_fwd_save_kernel<IdxT, false>;
   kern<<<M, kRowThreads, smem, stream>>>((const __nv_bfloat16*)logits, ld, (const IdxT*)targets, losses, stats,
-                                         (__nv_bfloat16*)copy, ld_copy, V, V_real, ignore_index, nullptr);
+                                         (__nv_bfloat16*)copy, ld_copy, V, V_real, ignore_index, strict, status);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
 int ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* stats,
-                void* copy, long long ld_copy, int M, int V, int V_real, int ignore_index, cudaStream_t stream) {
+                void* copy, long long ld_copy, int M, int V, int V_real, int ignore_index, int strict, int* status,
+                cudaStream_t stream) {
   if (M <= 0) return 0;
   if (V < 1 || V_real < 1 || V_real > V || ld < V || (reinterpret_cast<uintptr_t>(logits) & 1)) return 1;
   if (copy != nullptr && (ld_copy % 8 || ld_copy < (V + 7) / 8 * 8 || (reinterpret_cast<uintptr_t>(copy) & 15))) return 1;
   if (reinterpret_cast<uintptr_t>(stats) & 7) return 1;
   auto f = idx_is_64 ? ce_fwd_save_t<long long> : ce_fwd_save_t<int>;
-  return f(logits, ld, targets, losses, reinterpret_cast<float2*>(stats), copy, ld_copy, M, V, V_real, ignore_index,
-           stream);
+  return f(logits, ld, targets, losses, reinterpret_cast<float2*>(stats), copy, ld_copy, M, V, V_real, ignore_index, strict,
+           status, stream);
 }
 
 int ce_bwd(const void* x, const void* targets, int idx_is_64, const float* stats, const float* upstream, float scale,
-           void* grad, long long ld, int M, int V, int V_real, int ignore_index, cudaStream_t stream) {
+           void* grad, long long ld, int M, int V, int V_real, int ignore_index, int strict, cudaStream_t stream) {
   if (M <= 0) return 0;
   if (V < 1 || V_real < 1 || V_real > V || ld % 8 || ld < (V + 7) / 8 * 8 ||
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(grad)) & 15) || (reinterpret_cast<uintptr_t>(stats) & 7))
@@ -484,10 +499,10 @@ int ce_bwd(const void* x, const void* targets, int idx_is_64, const float* stats
   const float2* st = reinterpret_cast<const float2*>(stats);
   if (idx_is_64)
     ce_bwd_kernel<long long><<<M, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (const long long*)targets, st, upstream,
-                                                         scale, (__nv_bfloat16*)grad, ld, V, V_real, ignore_index);
+                                                         scale, (__nv_bfloat16*)grad, ld, V, V_real, ignore_index, strict);
   else
     ce_bwd_kernel<int><<<M, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (const int*)targets, st, upstream, scale,
-                                                   (__nv_bfloat16*)grad, ld, V, V_real, ignore_index);
+                                                   (__nv_bfloat16*)grad, ld, V, V_real, ignore_index, strict);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
@@ -513,13 +528,14 @@ int z2h_ce_fwd_bwd(void* logits, const void* targets, int idx_is_64, float* loss
                          write_grad, ignore_index, (cudaStream_t)stream);
 }
 int z2h_ce_fwd_save(const void* logits, long long ld, const void* targets, int idx_is_64, float* losses, float* stats,
-                    void* copy, long long ld_copy, int M, int V, int V_real, int ignore_index, void* stream) {
-  return z2h::ce_fwd_save(logits, ld, targets, idx_is_64, losses, stats, copy, ld_copy, M, V, V_real, ignore_index,
-                          (cudaStream_t)stream);
+                    void* copy, long long ld_copy, int M, int V, int V_real, int ignore_index, int strict, int* status,
+                    void* stream) {
+  return z2h::ce_fwd_save(logits, ld, targets, idx_is_64, losses, stats, copy, ld_copy, M, V, V_real, ignore_index, strict,
+                          status, (cudaStream_t)stream);
 }
 int z2h_ce_bwd(const void* x, const void* targets, int idx_is_64, const float* stats, const float* upstream, float scale,
-               void* grad, long long ld, int M, int V, int V_real, int ignore_index, void* stream) {
-  return z2h::ce_bwd(x, targets, idx_is_64, stats, upstream, scale, grad, ld, M, V, V_real, ignore_index,
+               void* grad, long long ld, int M, int V, int V_real, int ignore_index, int strict, void* stream) {
+  return z2h::ce_bwd(x, targets, idx_is_64, stats, upstream, scale, grad, ld, M, V, V_real, ignore_index, strict,
                      (cudaStream_t)stream);
 }
 int z2h_compact_rows(const void* src, long long ld, void* dst, int M, int N, void* stream) {

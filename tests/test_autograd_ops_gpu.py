@@ -89,6 +89,26 @@ def test_cross_entropy_of_the_largest_values(V):
         assert _rel(x.grad[[0, 2]] * 1.5, ref.grad[[0, 2]]) < BF16
 
 
+def test_cross_entropy_shows_a_label_out_of_range():
+    from zero_to_hero_b200.ops import _lib, functional as Z
+
+    _lib.check_status("cuda")
+    x = torch.randn(4, 33).bfloat16().cuda().requires_grad_()
+    for bad in (33, -1, 1 << 40):
+        t = torch.tensor([1, bad, 2, -100], device="cuda")
+        loss = Z.cross_entropy(x, t)
+        (grad,) = torch.autograd.grad(loss, x, retain_graph=True)
+        (again,) = torch.autograd.grad(loss, x, create_graph=True)
+        assert loss.isnan() and grad[1].isnan().all() and again[1].isnan().all()
+        with pytest.raises(RuntimeError, match="bad argument"):
+            _lib.check_status("cuda")
+    t = torch.tensor([1, 32, 0, -100], device="cuda")
+    assert torch.allclose(Z.cross_entropy(x, t), F.cross_entropy(x.float(), t), rtol=1e-5)
+    wide = torch.randn(4, 40).bfloat16().cuda()  # multiples of 8: such a row has always counted as ignored
+    assert Z.cross_entropy(wide, torch.tensor([1, 40, 2, -1], device="cuda")).isfinite()
+    _lib.check_status("cuda")
+
+
 @pytest.mark.parametrize("M,K,N,bias", [(1, 8, 1, True), (300, 384, 65, True), (130, 64, 127, False),
                                         (2048, 64, 257, True), (33, 768, 50257, False)])
 def test_linear_of_any_width(M, K, N, bias):

@@ -396,7 +396,8 @@ class _CrossEntropy(torch.autograd.Function):
 class _CrossEntropySaved(torch.autograd.Function):
     """The same over bf16 logits whose rows are tight in memory, any vocabulary: one pass forward that keeps
     a copy of the logits (the caller's may change before the backward), one pass backward that rounds the
-    gradient once. `skip_ignored`: the mean is over the targets that are not ignored."""
+    gradient once. `skip_ignored`: the mean is over the targets that are not ignored, and a label that names
+    neither a class nor -100 makes it NaN (and shows in the status word)."""
 
     @staticmethod
     def forward(ctx, logits, targets, v_real, skip_ignored):
@@ -407,7 +408,7 @@ class _CrossEntropySaved(torch.autograd.Function):
         copy = None
         if ctx.needs_input_grad[0]:
             copy = torch.empty(M, (V + 7) // 8 * 8, device=logits.device, dtype=torch.bfloat16)
-        N.ce_fwd_save(logits, targets, losses, stats, copy, v_real)
+        N.ce_fwd_save(logits, targets, losses, stats, copy, v_real, strict=skip_ignored)
         count = (targets != -100).sum().float() if skip_ignored else None
         if copy is not None:
             ctx.save_for_backward(copy, targets, stats, count)
@@ -425,13 +426,15 @@ class _CrossEntropySaved(torch.autograd.Function):
             x = ctx.logits if skipping and ctx.logits._version == ctx.version else copy
             x = x[:, :v_real].float()
             valid = ((targets >= 0) & (targets < v_real)).float()
+            if skipping:
+                valid = valid.masked_fill((valid == 0) & (targets != -100), math.nan)
             hit = (targets[:, None] == torch.arange(v_real, device=x.device)).float()
             p = x.softmax(1) if skipping else torch.exp(x - stats[:, :1] - stats[:, 1:])
             grad = F.pad((p - hit) * valid[:, None], (0, V - v_real))
             return (grad * (g / count if skipping else g / M)).bfloat16(), None, None, None
         grad = torch.empty_like(copy)
         up = g / count if skipping else g
-        N.ce_bwd(copy, targets, stats, up.reshape(1), 1.0 if skipping else 1.0 / M, grad, V, v_real)
+        N.ce_bwd(copy, targets, stats, up.reshape(1), 1.0 if skipping else 1.0 / M, grad, V, v_real, strict=skipping)
         return grad[:, :V], None, None, None
 
 

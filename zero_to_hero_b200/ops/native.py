@@ -35,9 +35,9 @@ _sigs = {
     "z2h_ce_fwd_bwd": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_longlong,
                        c_float, c_int, c_int, c_void_p],
     "z2h_ce_fwd_save": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int,
-                        c_int, c_int, c_void_p],
+                        c_int, c_int, c_int, c_void_p, c_void_p],
     "z2h_ce_bwd": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, c_longlong, c_int, c_int, c_int,
-                   c_int, c_void_p],
+                   c_int, c_int, c_void_p],
     "z2h_compact_rows": [c_void_p, c_longlong, c_void_p, c_int, c_int, c_void_p],
     "z2h_pdl_scope": [c_int],
     "z2h_relu": [c_void_p, c_longlong, c_void_p],
@@ -147,23 +147,24 @@ def ce_fwd_bwd(logits, targets, losses, v_real, grad_scale, write_grad=True, ign
 CE_SAVE_MAX_COLUMNS = 57_300  # a row of logits lies in shared memory, two rows to an SM
 
 
-def ce_fwd_save(logits, targets, losses, stats, copy, v_real, ignore_index=-100):
+def ce_fwd_save(logits, targets, losses, stats, copy, v_real, ignore_index=-100, strict=False):
     """Losses of the rows of `logits` [M, V] (bf16, unit inner stride, any pitch) and their maxima and
     logarithms of the sums of exp(x - maximum) (`stats`, fp32 [M, 2]); `copy` ([M, >= V] on a pitch of a
-    multiple of 8, or None) receives the logits for `ce_bwd`."""
+    multiple of 8, or None) receives the logits for `ce_bwd`. `strict`: a label that is neither a class nor
+    `ignore_index` gives NaN and "bad argument" in the status word instead of counting as ignored."""
     M, V = logits.shape
     assert stats.shape == (M, 2) and stats.dtype == torch.float32 and stats.is_contiguous()
     _check(_f("z2h_ce_fwd_save")(ptr(logits), max(logits.stride(0), V) if M == 1 else logits.stride(0), ptr(targets),
                                  _is64(targets), ptr(losses), ptr(stats), ptr(copy),
-                                 0 if copy is None else copy.stride(0), M, V, v_real, ignore_index, stream_ptr()),
-           "ce_fwd_save")
+                                 0 if copy is None else copy.stride(0), M, V, v_real, ignore_index, int(strict),
+                                 ptr(_lib.status_word(logits.device)), stream_ptr()), "ce_fwd_save")
 
 
-def ce_bwd(copy, targets, stats, upstream, scale, grad, V, v_real, ignore_index=-100):
+def ce_bwd(copy, targets, stats, upstream, scale, grad, V, v_real, ignore_index=-100, strict=False):
     """grad = (softmax - onehot) * scale * upstream[0]; `copy` and `grad` share one pitch."""
     assert copy.stride(0) == grad.stride(0) and upstream.dtype == torch.float32
     _check(_f("z2h_ce_bwd")(ptr(copy), ptr(targets), _is64(targets), ptr(stats), ptr(upstream), scale, ptr(grad),
-                            copy.stride(0), copy.shape[0], V, v_real, ignore_index, stream_ptr()), "ce_bwd")
+                            copy.stride(0), copy.shape[0], V, v_real, ignore_index, int(strict), stream_ptr()), "ce_bwd")
 
 
 def compact_rows(src, dst):
