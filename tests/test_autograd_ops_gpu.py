@@ -109,6 +109,41 @@ def test_cross_entropy_shows_a_label_out_of_range():
     _lib.check_status("cuda")
 
 
+# what the graph keeps: freed by the backward even while the loss lives on, seen by saved-tensor hooks, and right
+# for a second derivative after the caller has changed its logits
+@pytest.mark.parametrize("V", (1001, 1008))
+def test_cross_entropy_keeps_its_logits_in_the_graph(V):
+    import weakref
+
+    from zero_to_hero_b200.ops import functional as Z
+
+    g = torch.Generator().manual_seed(V)
+    x = torch.randn(64, V, generator=g).bfloat16().cuda().requires_grad_()
+    t = torch.randint(0, V, (64,), generator=g).cuda()
+    before = torch.cuda.memory_allocated()
+    logits = x * 1.0
+    inner, packed = weakref.ref(logits), []
+    with torch.autograd.graph.saved_tensors_hooks(lambda s: packed.append(s.numel()) or s, lambda s: s):
+        loss = Z.cross_entropy(logits, t)
+    assert sum(n >= 64 * V for n in packed) == 1
+    del logits
+    assert inner() is None  # the graph holds its own copy only
+    loss.backward()
+    x.grad = None
+    assert torch.cuda.memory_allocated() - before < 64 * V  # `loss` is alive, the copy (two bytes each) is not
+    d = x.detach().double().requires_grad_()
+    logits = x * 1.0
+    loss, ref = Z.cross_entropy(logits, t), F.cross_entropy(d, t)
+    with torch.no_grad():
+        logits.zero_()
+    scale = torch.ones((), device="cuda", requires_grad=True)  # a graph of the backward for both kinds of width
+    (first,) = torch.autograd.grad(loss * scale, x, create_graph=True)
+    first.float().square().sum().backward()
+    (want,) = torch.autograd.grad(ref, d, create_graph=True)
+    want.square().sum().backward()
+    assert _rel(first, want) < BF16 and _rel(x.grad, d.grad) < 4 * BF16
+
+
 @pytest.mark.parametrize("M,K,N,bias", [(1, 8, 1, True), (300, 384, 65, True), (130, 64, 127, False),
                                         (2048, 64, 257, True), (33, 768, 50257, False)])
 def test_linear_of_any_width(M, K, N, bias):

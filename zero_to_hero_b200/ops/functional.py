@@ -396,7 +396,8 @@ class _CrossEntropy(torch.autograd.Function):
 class _CrossEntropySaved(torch.autograd.Function):
     """The same over bf16 logits whose rows are tight in memory, any vocabulary: one pass forward that keeps
     a copy of the logits (the caller's may change before the backward), one pass backward that rounds the
-    gradient once. `skip_ignored`: the mean is over the targets that are not ignored, and a label that names
+    gradient once. The copy is an output beside the loss: saved like any tensor and freed with the graph, and
+    what a second derivative goes through. `skip_ignored`: the mean is over the targets that are not ignored, and a label that names
     neither a class nor -100 makes it NaN (and shows in the status word)."""
 
     @staticmethod
@@ -406,6 +407,7 @@ class _CrossEntropySaved(torch.autograd.Function):
         losses = torch.empty(M, device=logits.device, dtype=torch.float32)
         stats = torch.empty(M, 2, device=logits.device, dtype=torch.float32)
         copy = None
+        ctx.set_materialize_grads(False)
         if ctx.needs_input_grad[0]:
             copy = torch.empty(M, (V + 7) // 8 * 8, device=logits.device, dtype=torch.bfloat16)
         N.ce_fwd_save(logits, targets, losses, stats, copy, v_real, strict=skip_ignored)
@@ -413,29 +415,30 @@ class _CrossEntropySaved(torch.autograd.Function):
         if copy is not None:
             ctx.save_for_backward(copy, targets, stats, count)
             ctx.meta = (M, V, v_real)
-            # a second derivative goes through the caller's logits themselves
-            ctx.logits, ctx.version = (logits, logits._version) if skip_ignored else (None, 0)
-        return losses.mean() if count is None else losses.sum() / count
+        return (losses.mean() if count is None else losses.sum() / count), copy
 
     @staticmethod
-    def backward(ctx, g):
+    def backward(ctx, g, g_copy):
         copy, targets, stats, count = ctx.saved_tensors
         M, V, v_real = ctx.meta
         skipping = count is not None
+        if g_copy is not None:  # a second derivative, on its way to the logits
+            g_copy = g_copy[:, :V]
+        if g is None:
+            return g_copy, None, None, None
         if torch.is_grad_enabled() and (g.requires_grad or skipping):  # a graph of this backward is wanted
-            x = ctx.logits if skipping and ctx.logits._version == ctx.version else copy
-            x = x[:, :v_real].float()
+            x = copy[:, :v_real].float()
             valid = ((targets >= 0) & (targets < v_real)).float()
             if skipping:
                 valid = valid.masked_fill((valid == 0) & (targets != -100), math.nan)
             hit = (targets[:, None] == torch.arange(v_real, device=x.device)).float()
-            p = x.softmax(1) if skipping else torch.exp(x - stats[:, :1] - stats[:, 1:])
-            grad = F.pad((p - hit) * valid[:, None], (0, V - v_real))
-            return (grad * (g / count if skipping else g / M)).bfloat16(), None, None, None
+            grad = F.pad((x.softmax(1) - hit) * valid[:, None], (0, V - v_real))
+            grad = (grad * (g / count if skipping else g / M)).bfloat16()
+            return grad if g_copy is None else grad + g_copy, None, None, None
         grad = torch.empty_like(copy)
         up = g / count if skipping else g
         N.ce_bwd(copy, targets, stats, up.reshape(1), 1.0 if skipping else 1.0 / M, grad, V, v_real, strict=skipping)
-        return grad[:, :V], None, None, None
+        return grad[:, :V] if g_copy is None else grad[:, :V] + g_copy, None, None, None
 
 
 def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, v_real: int | None = None) -> torch.Tensor:
@@ -448,10 +451,10 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, v_real: int | Non
                  and t.shape[0] == x.shape[0] and x.is_contiguous())
         if V % 8 == 0:
             if tight and t.dtype in (torch.int64, torch.int32):
-                return _CrossEntropySaved.apply(x, t, v_real, False)
+                return _CrossEntropySaved.apply(x, t, v_real, False)[0]
             return _CrossEntropy.apply(x, t, v_real)
         if tight and t.dtype == torch.int64 and t.device == x.device and not _transformed():
-            return _CrossEntropySaved.apply(x, t, v_real, True)
+            return _CrossEntropySaved.apply(x, t, v_real, True)[0]
     if _native(logits):
         FALLBACK_COUNTS["cross_entropy"] += 1
     return F.cross_entropy(logits.reshape(-1, V)[:, :v_real].float(), targets.reshape(-1))
