@@ -1,6 +1,6 @@
 // Activations of the MLP outside the GEMMs: ReLU, and the backward of GELU (dx = dy * gelu'(x) for a saved
-// bf16 x) and ReLU (dx = dy where the output is positive), with the column sums of dx (the bias gradient of
-// the layer that produced x) added up on the way.
+// bf16 x) and ReLU (dx = 0 where the output is zero or less, dy elsewhere, at a NaN too), with the column
+// sums of dx (the bias gradient of the layer that produced x) added up on the way.
 //
 // Bound by memory: 6 bytes an element. A CTA takes 256 columns (32 lanes x 8) of a slab of rows, one row
 // per warp; a thread keeps its 8 column sums in registers over the slab, the 8 warps fold theirs in
@@ -42,7 +42,7 @@ act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __rest
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 a = unpack_bf16x2(gw[j]), b = unpack_bf16x2(xw[j]);
-        ow[j] = RELU ? pack_bf16x2(b.x > 0.f ? a.x : 0.f, b.y > 0.f ? a.y : 0.f)
+        ow[j] = RELU ? pack_bf16x2(b.x <= 0.f ? 0.f : a.x, b.y <= 0.f ? 0.f : a.y)
                      : pack_bf16x2(a.x * gelu_tanh_grad_exact(b.x), a.y * gelu_tanh_grad_exact(b.y));
         const float2 q = unpack_bf16x2(ow[j]);  // the sums are those of the stored values
         s[2 * j] += q.x;

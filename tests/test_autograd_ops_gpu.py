@@ -217,3 +217,22 @@ def test_odd_widths_that_the_kernels_do_not_compute_keep_the_library():
     for bad in ((x, w[:, :32]), (x, w.cpu()), (x, w, torch.zeros(6).cuda()), (x, w, torch.zeros(7))):
         with pytest.raises(RuntimeError):  # F.linear's own refusal, on the host
             Z.linear(*bad)
+
+
+@pytest.mark.parametrize("M,N", [(1, 8), (70, 264)])
+def test_relu_and_its_backward(M, N):
+    from zero_to_hero_b200.ops import native
+
+    x = torch.randn(M, N, generator=torch.Generator().manual_seed(M)).bfloat16().cuda()
+    x[0, :6] = torch.tensor([0.0, -0.0, torch.nan, torch.inf, -torch.inf, 1e-40])
+    dy = torch.randn(M, N, generator=torch.Generator().manual_seed(N)).bfloat16().cuda()
+    ref = x.clone().requires_grad_()
+    y = F.relu(ref)
+    y.backward(dy)
+    out = x.clone()
+    native.relu_(out)
+    dx, db = torch.empty_like(dy), torch.zeros(N, device="cuda")
+    native.relu_bwd(dy, out, dx, db)
+    assert torch.equal(out.nan_to_num(), y.detach().nan_to_num()) and torch.equal(out.isnan(), y.isnan())
+    assert torch.equal(dx, ref.grad)
+    assert torch.allclose(db.double(), ref.grad.double().sum(0), rtol=1e-5, atol=1e-5 * M ** 0.5)

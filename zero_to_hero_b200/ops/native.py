@@ -185,7 +185,7 @@ def relu_(x):
 
 
 def relu_bwd(dy, out, dx, db=None):
-    """dx = dy where out > 0, else 0, over tight bf16 [M, N]; `db` (fp32 [N]) += column sums of dx."""
+    """dx = 0 where out <= 0, else dy (at a NaN too), over tight bf16 [M, N]; `db` (fp32 [N]) += column sums of dx."""
     M, N = out.shape
     _check(_f("z2h_relu_bwd")(ptr(dy), ptr(out), ptr(dx), ptr(db), M, N, stream_ptr()), "relu_bwd")
 
