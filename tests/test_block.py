@@ -100,3 +100,24 @@ def test_block_matches_the_single_ops(make, B, T, kw, bf16):
     m(X.cuda(), Y.cuda())[1].backward()
     assert all(p.grad is None for p in frozen)
     assert all(p.grad is not None for p in m.parameters() if p.requires_grad)
+
+
+# The derivative of the activation by itself: a hidden unit's input is its bias alone, every unit gets the
+# gradient 16, and the bias gradient adds the same number once per token.
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", (32, 31))
+def test_block_gelu_derivative_is_exact(T):
+    block = _gpt2(layers=1).transformer.h[0]
+    with torch.no_grad():
+        block.mlp.c_fc.weight.zero_()
+        block.mlp.c_fc.bias.copy_(torch.linspace(-5, 5, 512).bfloat16())
+        block.mlp.c_proj.weight.fill_(0.125)
+    block = block.cuda()
+    out = block(torch.randn(1, T, 128).bfloat16().cuda())
+    assert "_Block" in type(out.grad_fn).__name__
+    out.backward(torch.ones_like(out))
+    b = block.mlp.c_fc.bias.detach().double().requires_grad_()
+    nn.functional.gelu(b, approximate="tanh").sum().backward()
+    want = 16 * T * b.grad
+    # 512 numbers rounded to 8 bits each, and an error of 1e-6 in the derivative
+    assert ((block.mlp.c_fc.bias.grad.double() - want).abs() <= 2.0 ** -8 * want.abs() + 16 * T * 2e-6).all()

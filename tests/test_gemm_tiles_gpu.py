@@ -4,7 +4,7 @@ import torch
 import torch.nn.functional as F
 
 pytestmark = pytest.mark.gpu
-BF16 = 2.0 ** -8  # a rounding to bf16 is off by at most 2^-9; two meet where a second one follows
+BF16 = 2.0 ** -8  # a rounding to bf16 is off by at most this share of the value
 
 
 def _rel(a, b):
