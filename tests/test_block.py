@@ -121,3 +121,18 @@ def test_block_gelu_derivative_is_exact(T):
     want = 16 * T * b.grad
     # 512 numbers rounded to 8 bits each, and an error of 1e-6 in the derivative
     assert ((block.mlp.c_fc.bias.grad.double() - want).abs() <= 2.0 ** -8 * want.abs() + 16 * T * 2e-6).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", (_gpt2, _char))
+def test_block_gradients_do_not_share_memory(make):
+    m = make().cuda()
+    X = torch.randint(0, 60, (2, 33)).cuda()
+    m(X, X)[1].backward()
+    for b in m.transformer.h if make is _gpt2 else m.blocks:
+        for n, p in b.named_parameters():
+            size = p.grad.untyped_storage().nbytes()
+            if ".heads." in n:  # row blocks of one matrix, whose gradient is one product
+                assert size == 3 * p.shape[1] ** 2 * 4
+            else:
+                assert size == p.numel() * 4

@@ -122,8 +122,13 @@ class _Block(torch.autograd.Function):
         def buf(*shape, dtype=torch.bfloat16):
             return torch.empty(*shape, device=dev, dtype=dtype)
 
-        # fp32 gradients of all parameters in one buffer of zeros, laid out like the bf16 copies
-        g, g_qkv = _split(torch.zeros(flat.numel(), device=dev, dtype=torch.float32), named, sizes, C)
+        # fp32 gradients, zeroed together; each a tensor of its own, because they become the parameters' `.grad`: as
+        # views of one buffer any of them would keep, and a saved one would contain, those of the whole block
+        new, f32, g = flat.new_empty, torch.float32, dict.fromkeys(_ORDER)
+        for n, size in zip(named, sizes):
+            g[n] = new((_SHAPES[n][0] * C, _SHAPES[n][1] * C) if n in _SHAPES else size, dtype=f32)
+        g_qkv = new((3 * C, C), dtype=f32)
+        torch._foreach_zero_([g_qkv, *(g[n] for n in named)])
         w, w_qkv = _split(flat, named, sizes, C)
         needs = dict(zip(_ORDER, need))
 
