@@ -127,6 +127,18 @@ def test_generate_past_the_context_window_and_sampling_seeds():
     assert m.generate(X.int(), 2, generator=g).shape == (2, 22) and m.generate(X, 0) is X
 
 
+@pytest.mark.gpu
+def test_status_word_made_by_generate_can_be_reset_outside(monkeypatch):
+    from zero_to_hero_b200.ops import _lib
+
+    monkeypatch.setattr(_lib, "_status", {})
+    _model().cuda().generate(torch.zeros(1, 1, dtype=torch.int64, device="cuda"), 1)
+    _lib.status_word("cuda").fill_(6)
+    with pytest.raises(RuntimeError, match="timeout in an intra-CTA wait"):
+        _lib.check_status("cuda")
+    _lib.check_status("cuda")
+
+
 # the top-k select: values that crowd into one first digit, ties, both signs of zero, -inf, one row in
 # shared memory and one too long for it
 @pytest.mark.gpu

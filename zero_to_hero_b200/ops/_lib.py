@@ -82,7 +82,8 @@ def status_word(device: torch.device | int | None = None) -> torch.Tensor:
     """Per-device int32 status word that bounded device-side waits write to (0 == ok)."""
     idx = torch.cuda.current_device() if device is None else torch.device(device).index or 0
     if idx not in _status:
-        _status[idx] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{idx}")
+        with torch.inference_mode(False):  # the first use may be in generate(); the word is reset outside it, too
+            _status[idx] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{idx}")
     return _status[idx]
 
 
