@@ -139,6 +139,23 @@ def test_status_word_made_by_generate_can_be_reset_outside(monkeypatch):
     _lib.check_status("cuda")
 
 
+@pytest.mark.gpu
+def test_generate_raises_what_a_kernel_reported():
+    from zero_to_hero_b200.ops import _lib
+
+    m = _model().cuda()
+    X = torch.zeros(2, 3, dtype=torch.int64, device="cuda")
+    _lib.check_status("cuda")
+    want = m.generate(X, 4, top_k=1)
+    _lib.status_word("cuda").fill_(6)  # what an expired wait leaves
+    with pytest.raises(RuntimeError, match="timeout in an intra-CTA wait"):
+        m.generate(X, 4, top_k=1)
+    assert torch.equal(m.generate(X, 4, top_k=1), want)
+    with pytest.raises(RuntimeError, match="bad argument"):
+        m.generate(X + 101, 4, top_k=1)  # one past the vocabulary: clamped, and reported
+    _lib.check_status("cuda")
+
+
 # the top-k select: values that crowd into one first digit, ties, both signs of zero, -inf, one row in
 # shared memory and one too long for it
 @pytest.mark.gpu

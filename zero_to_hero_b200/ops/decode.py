@@ -237,7 +237,8 @@ def generate(model, X: torch.Tensor, max_new_tokens: int, temperature: float, to
              generator: torch.Generator | None) -> torch.Tensor | None:
     """`GPT2.generate` with cached keys and values; None where the memory for it is not there (nothing
     has been sampled then). Positions are absolute, so once the sequence outgrows the context every
-    token shifts all of them: the window is then run through the batched pass again for each token."""
+    token shifts all of them: the window is then run through the batched pass again for each token. Raises when a
+    kernel has reported a failure (an expired wait, a token out of range)."""
     from .sampling import sample_next
 
     B, T0 = X.shape
@@ -255,4 +256,8 @@ def generate(model, X: torch.Tensor, max_new_tokens: int, temperature: float, to
             session.prefill(tokens[:, first:T - 1])
         logits = session.step(tokens[:, T - 1], T - 1 - first)
         sample_next(logits, temperature, top_k, generator, out=tokens[:, T])
+    if not torch.cuda.is_current_stream_capturing():
+        # A wait between CTAs that ran out leaves the step's results wrong and says so in the status word alone. Read
+        # once a call, after the last launch: raises, as the engine does when it reads a loss.
+        _lib.check_status(session.device)
     return torch.cat((X, tokens[:, T0:]), dim=1)
