@@ -72,6 +72,19 @@ def test_only_plain_models_take_the_decode_kernel():
     assert changed(lambda m: m.train()) and changed(lambda m: None, dropout=0.1)
 
 
+def test_shapes_that_the_kernel_refuses_keep_the_general_path(monkeypatch):
+    asked = []
+
+    def epochs(n, C, layers):  # a device where eight wide sequences do not fit
+        asked.append((n, C, layers))
+        return 0 if n * C > 8 * 1024 else 5 * layers
+
+    monkeypatch.setattr(decode, "_f", lambda name: {"z2h_decode_epochs": epochs}[name])
+    assert decode.group_sizes(1) == [1] and decode.group_sizes(8) == [8] and decode.group_sizes(19) == [8, 8, 3]
+    assert decode.kernel_takes(19, 1024, 2) and sorted(asked) == [(3, 1024, 2), (8, 1024, 2)]
+    assert decode.kernel_takes(3, 2048, 2) and not decode.kernel_takes(8, 2048, 2) and not decode.kernel_takes(11, 2048, 2)
+
+
 def _general(m, X):
     """Logits after each prompt prefix, through the module's forward."""
     return torch.stack([m(X[:, :t][:, -m.config.block_size:])[0][:, -1].float() for t in range(1, X.shape[1] + 1)], 1)
@@ -125,6 +138,17 @@ def test_generate_past_the_context_window_and_sampling_seeds():
     assert torch.equal(again, m.generate(X, 12, temperature=0.9, top_k=7))
     g = torch.Generator("cuda").manual_seed(4)
     assert m.generate(X.int(), 2, generator=g).shape == (2, 22) and m.generate(X, 0) is X
+
+
+@pytest.mark.gpu
+def test_generate_where_the_kernel_does_not_fit(monkeypatch):
+    m = _model().cuda()
+    X = torch.zeros(2, 3, dtype=torch.int64, device="cuda")
+    assert decode.supports(m, X)
+    want = m.generate(X, 4, top_k=1)
+    monkeypatch.setattr(decode, "_fns", {**decode._fns, "z2h_decode_epochs": lambda n, C, layers: 0})
+    assert not decode.supports(m, X)
+    assert torch.equal(m.generate(X, 4, top_k=1), want)
 
 
 @pytest.mark.gpu

@@ -129,7 +129,18 @@ def supports(model, X: torch.Tensor) -> bool:
         return False
     if torch.is_autocast_enabled() or torch.compiler.is_compiling() or X.device.index != torch.cuda.current_device():
         return False
-    return plain_model(model) and model.lm_head.weight.device == X.device
+    return plain_model(model) and model.lm_head.weight.device == X.device and \
+        kernel_takes(X.shape[0], cfg.emb_dim, cfg.num_layers)
+
+
+def group_sizes(batch: int) -> list[int]:
+    """Sequences of the launches that a step of `batch` sequences takes."""
+    return [min(MAX_BATCH, batch - b0) for b0 in range(0, batch, MAX_BATCH)]
+
+
+def kernel_takes(batch: int, C: int, layers: int) -> bool:
+    """The kernel's own rule, which depends on the device (2048 columns need 128 SMs)."""
+    return all(_f("z2h_decode_epochs")(n, C, layers) != 0 for n in set(group_sizes(batch)))
 
 
 def expected_shapes(cfg) -> dict[str, tuple[int, ...]]:
@@ -153,8 +164,8 @@ class DecodeSession:
         self._pack([(params[n], at) for n, at in self.offsets.items()])
         self.shapes = {n: tuple(p.shape) for n, p in params.items()}
         self.groups = []
-        for b0 in range(0, batch, MAX_BATCH):
-            n = min(MAX_BATCH, batch - b0)
+        for i, n in enumerate(group_sizes(batch)):
+            b0 = i * MAX_BATCH
             kv = torch.empty(self.L, 2, n, max_len, self.C, device=self.device, dtype=torch.bfloat16)
             scratch = torch.zeros(_f("z2h_decode_scratch_bytes")(n, self.C, self.H), device=self.device, dtype=torch.uint8)
             epochs = _f("z2h_decode_epochs")(n, self.C, self.L)
