@@ -417,6 +417,14 @@ __device__ __forceinline__ void layer_norm_rows(const Params& p, Smem* sm, const
   consumer_sync();
 }
 
+// The larger one, NaN if one is NaN (fmaxf drops it, and a warp or a key range of NaNs alone would then look
+// like one without keys).
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+  return m;
+}
+
 // One (sequence, head, key range): keys are dealt to the warps four at a time (8 lanes per key, 16
 // bytes each), 16 per warp and round, with all key and value loads of a round in flight together.
 __device__ __forceinline__ void attend(const Params& p, Smem* sm, int layer, uint32_t in_epoch, uint32_t out_epoch) {
@@ -482,12 +490,12 @@ __device__ __forceinline__ void attend(const Params& p, Smem* sm, int layer, uin
         d += __shfl_xor_sync(0xffffffffu, d, 2);
         d += __shfl_xor_sync(0xffffffffu, d, 4);
         sc[i] = base + i * (kWarps * 4) + warp * 4 + grp < k1 ? d : -INFINITY;
-        mr = fmaxf(mr, sc[i]);
+        mr = max_nan(mr, sc[i]);
       }
-      mr = fmaxf(mr, __shfl_xor_sync(0xffffffffu, mr, 8));
-      mr = fmaxf(mr, __shfl_xor_sync(0xffffffffu, mr, 16));
-      if (mr > -INFINITY) {  // warp-uniform: this warp has keys in the round
-        const float mn = fmaxf(m, mr), keep = ex2_fast(m - mn);
+      mr = max_nan(mr, __shfl_xor_sync(0xffffffffu, mr, 8));
+      mr = max_nan(mr, __shfl_xor_sync(0xffffffffu, mr, 16));
+      if (!(mr == -INFINITY)) {  // warp-uniform: this warp has keys in the round (or a NaN, which l and o take on)
+        const float mn = max_nan(m, mr), keep = ex2_fast(m - mn);
         m = mn;
         l *= keep;
 #pragma unroll
@@ -569,6 +577,8 @@ __device__ __forceinline__ void fold_attention(const Params& p, Smem* sm, uint8_
         o.y = o.y * f + __uint_as_float(v[1].y) * g;
         o.z = o.z * f + __uint_as_float(v[2].x) * g;
         o.w = o.w * f + __uint_as_float(v[2].y) * g;
+      } else {
+        l += __uint_as_float(v[0].y);  // 0, or NaN from keys of NaN
       }
     }
     *reinterpret_cast<uint2*>(xs + b * p.xs_stride + c * 2) =

@@ -119,6 +119,26 @@ def test_decode_matches_the_forward_pass(heads, layers, vocab, block, B, T, ln_b
     assert e_got <= 1.3 * e_mod + 1e-3, (float(e_got), float(e_mod))
 
 
+# NaN keys reach the result, wherever they lie: one among others, all keys of a warp (it takes four neighbours and
+# those 60 further on), a whole key range, the step's own. The sequence beside them stays clean.
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,first,count", [(1, 0, 1), (3, 0, 1), (5, 4, 1), (9, 4, 4), (64, 0, 1), (60, 8, 4), (61, 60, 1),
+                                           (900, 301, 1), (900, 100, 250), (900, 0, 899), (897, 780, 117)])
+def test_decode_keeps_nan(T, first, count):
+    m = _model(heads=2, layers=1, vocab=101, block=900).cuda()
+    X = torch.randint(0, 101, (2, T), generator=torch.Generator().manual_seed(T)).cuda()
+    with torch.inference_mode():
+        s = decode.DecodeSession(m, 2, T)
+        s.prefill(X[:, :T - 1])
+        clean = s.step(X[:, T - 1], T - 1).clone()
+        s.groups[0]["kv"][0, 0, 0, first:first + count, 70] = torch.nan  # a column of head 1
+        if first + count == T:  # the step's own key: a bias reaches it, and the other sequence's too
+            s.view("transformer.h.0.attn.c_attn.bias")[128 + 70] = torch.nan
+        got = s.step(X[:, T - 1], T - 1)
+    assert clean.isfinite().all() and got[0].isnan().all()
+    assert got[1].isnan().all() if first + count == T else torch.equal(got[1], clean[1])
+
+
 @pytest.mark.gpu
 def test_generate_past_the_context_window_and_sampling_seeds():
     m = _model(heads=2, layers=2, vocab=101, block=24).cuda()
