@@ -12,26 +12,35 @@ int gemm_get_algo() { return g_algo; }
 // drain. Narrow tiles are less efficient each, but where 256 columns leave SMs without a tile they finish
 // first. Measured at 256 / 128 / 64 columns, us: M1024 N768 K768 9.4 / 8.4 / 7.8, M1024 N2304 K768
 // 9.8 / 9.2 / 12.7, M2545 N1152 K384 8.0 / 9.2 / 10.9, M512 N384 K128 6.2 / 5.3 / 4.4.
-static int pick_bn(const GemmArgs& g) {
-  if (g_algo == 64 || g_algo == 128) return g_algo;
-  if (g_algo != 2 || g.split_k != 1 || g.max_ctas > 0) return 256;
-  const long long sms = sm_count_current_device(), kb = (g.K + 63) / 64, tm = (g.M + 127) / 128;
+static int pick_bn(long long M, long long N, long long K, long long sms) {
+  const long long kb = (K + 63) / 64, tm = (M + 127) / 128;
   int best = 256;
   long long best_cost = 0;
   for (int bn = 256; bn >= 64; bn /= 2) {
-    const long long waves = (tm * ((g.N + bn - 1) / bn) + sms - 1) / sms, mma = 4 * (44 + bn / 2);
+    const long long waves = (tm * ((N + bn - 1) / bn) + sms - 1) / sms, mma = 4 * (44 + bn / 2);
     const long long cost = waves * (kb * (mma < 400 ? 400 : mma) + 1500 + 4 * bn);
     if (bn == 256 || cost < best_cost) { best = bn; best_cost = cost; }
   }
   return best;
 }
 
-// Whether pairs of SMs would need another wave for a few 256 x 256 tiles where single SMs do not, as for 808
-// rows (4 tiles of 256, 7 of 128) by 4800 columns: 21.4 us in pairs, 14.2 us without (K 1600).
-static bool pairs_spill_over(const GemmArgs& g) {
-  const long long sms = sm_count_current_device(), tn = (g.N + 255) / 256;
-  const long long pairs = ((g.M + 255) / 256 * tn + sms / 2 - 1) / (sms / 2);
-  return g.split_k == 1 && ((g.M + 127) / 128 * tn + sms - 1) / sms < pairs;
+// Whether pairs of SMs would need another wave for a few 256 x 256 tiles where single SMs do not. A wave of
+// pairs is the shorter one (0.8 of a wave of single SMs at K 768), so one wave less pays while there are few:
+// single / pairs, us, at 2 waves of pairs (M808 N4800 K1600) 14.3 / 22.2, 3 (M1920 N4800 K768) 16.5 / 19.9, 6
+// (M2331 N9600 K768) 32.4 / 33.1; but at 8 (M640 N50264 K768) 66.7 / 58.8, at 27 (M2331 N50264 K768) 211 / 176.
+// A short contraction is bound by its stores, alike in both: K 192 at 27 waves 150 to 161 / 160.
+static bool pairs_spill_over(long long M, long long N, long long K, long long sms) {
+  const long long tn = (N + 255) / 256;
+  const long long pairs = ((M + 255) / 256 * tn + sms / 2 - 1) / (sms / 2);
+  return ((M + 127) / 128 * tn + sms - 1) / sms < pairs && (pairs <= 6 || K <= 192);
+}
+
+// The kernel for a product without split K on `sms` SMs: 2 = CTA pairs, else the tile width of the one-CTA
+// kernel.
+static int pick_kernel(long long M, long long N, long long K, long long sms) {
+  const long long tiles = (M + 255) / 256 * ((N + 255) / 256);
+  if (M >= 256 && tiles >= sms / 2 && !pairs_spill_over(M, N, K, sms)) return 2;
+  return pick_bn(M, N, K, sms);
 }
 
 int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
@@ -59,16 +68,16 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
   if ((reinterpret_cast<uintptr_t>(g.residual) & 15) || (reinterpret_cast<uintptr_t>(g.aux_out) & 15) ||
       (reinterpret_cast<uintptr_t>(g.aux_in) & 15))
     return 1;
-  {
+  int kernel = g_algo == 0 ? 256 : g_algo == 1 ? (g.M >= 256 ? 2 : 256) : g_algo;
+  if (g_algo == 2) {
     const bool stream_k = g.split_k <= 0 && g.epi == kEpiAtomicAdd;  // fills every SM whatever the tile count
-    const long long tiles256 = (long long)((g.M + 255) / 256) * ((g.N + 255) / 256) * (g.split_k < 1 ? 1 : g.split_k);
     // split-K and stream-K launches always take the pair kernel: it measured faster at every factor
-    const bool pair = g_algo == 1 ? g.M >= 256
-                                  : (g_algo == 2 && g.M >= 256 && (stream_k || g.split_k > 1 ||
-                                                  (tiles256 >= sm_count_current_device() / 2 && !pairs_spill_over(g))));
-    if (pair) return gemm_bf16_pair(g, stream);
+    if (stream_k || g.split_k > 1) kernel = g.M >= 256 ? 2 : 256;
+    else kernel = pick_kernel(g.M, g.N, g.K, sm_count_current_device());
+    if (kernel != 2 && g.max_ctas > 0) kernel = 256;
   }
-  switch (pick_bn(g)) {
+  switch (kernel) {
+    case 2: return gemm_bf16_pair(g, stream);
     case 64: return gemm_bf16_narrow64(g, stream);
     case 128: return gemm_bf16_narrow128(g, stream);
     default: return launch_onecta<256>(g, stream);
@@ -84,6 +93,8 @@ extern "C" int z2h_gemm_trace_read(long long* host_out) {
 #endif
 extern "C" void z2h_gemm_set_algo(int algo) { z2h::gemm_set_algo(algo); }
 extern "C" void z2h_gemm_set_fixup(int on) { z2h::gemm_set_fixup(on); }
+// Which kernel the automatic choice takes for a product without split K (see pick_kernel).
+extern "C" int z2h_gemm_pick_kernel(int M, int N, int K, int sms) { return z2h::pick_kernel(M, N, K, sms); }
 extern "C" int z2h_gemm_get_algo() { return z2h::gemm_get_algo(); }
 namespace z2h {
 namespace {
