@@ -9,9 +9,11 @@
 // latency and the prologue of every kernel at each of the ~310 boundaries of a micro-step.
 // Measured inside CUDA graphs (two runs each way on one box, the runs of one side 0.3 % apart): a training
 // step of the 2-layer, 128-wide model 503 -> 488 us, of the 124M model 35.1 -> 34.7 ms, of the 350M model
-// 50.0 -> 49.3 ms, evaluation of 16 x 1024 tokens 5.85 -> 5.81 ms, of 4 x 256 tokens 945 -> 949 us. (An
-// earlier state of the kernels was 0.8 % slower with it.) So the engine asks for it, through the launching
-// thread's pdl_scope, for training steps and for evaluations of 4096 tokens and more; elsewhere it is off.
+// 50.0 -> 49.3 ms. Evaluations, replays of both graphs in turn: 16 x 512 tokens 3.04 -> 2.91 ms (124M), 8 x 1024
+// 3.13 -> 3.02, 4 x 1024 1.77 -> 1.67, 16 x 1024 5.70 -> 5.68; of 512 to 2,048 tokens between 4.9 % slower and 10 %
+// faster. (An earlier state of the kernels was 0.8 % slower with it.) So the engine asks for it, through the
+// launching thread's pdl_scope, for training steps and for evaluations of 4096 tokens and more
+// (PDL_EVAL_TOKENS); elsewhere it is off.
 // Z2H_PDL=1 or 0 in the environment decides for all launches.
 #pragma once
 #include <cuda_runtime.h>

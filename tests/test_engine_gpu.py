@@ -361,3 +361,40 @@ def test_deterministic_mode_repeats_training_bit_for_bit(dropout):
     assert a[3][-1][0] == pytest.approx(plain[3][-1][0], abs=2e-3)
     assert (a[0] - plain[0]).abs().max().item() < 2.5e-3 * 3
     _lib.check_status()
+
+
+# Dependent launch moves the start of every kernel ahead of the end of the one before: what a kernel reads too
+# early shows as other bits. Reproducible sums, weight gradients on the side stream, with and without dropout.
+@pytest.mark.parametrize("dropout", (0.0, 0.2))
+def test_dependent_launch_changes_no_bit(dropout, monkeypatch):
+    import contextlib
+
+    from zero_to_hero_b200 import engine as E
+    from zero_to_hero_b200.ops import native as N
+
+    monkeypatch.setattr(E, "PDL_EVAL_TOKENS", 1)
+    scopes = []
+
+    def scope(on, real=N.pdl_scope):
+        scopes.append(on)
+        return real(on)
+
+    def run():
+        cfg = _cfg()
+        cfg.train.deterministic = cfg.train.overlap_wgrad = cfg.train.use_cuda_graph = True
+        cfg.model.dropout = dropout
+        eng = E.GPT2TrainEngine(cfg, "cuda", seed=1)
+        g = torch.Generator().manual_seed(7)
+        seen = []
+        for _ in range(6):
+            batches = _batches(g)
+            eng.train_step(batches, lr=1e-3)
+            seen += [torch.tensor(eng.read_loss()), eng.eval_losses(*batches[0]).clone().cpu(),
+                     eng.eval_losses(batches[1][0][:3, :77], batches[1][1][:3, :77]).clone().cpu()]
+        return seen + [eng.p32.cpu(), eng.m.cpu(), eng.v.cpu()]
+
+    monkeypatch.setattr(N, "pdl_scope", scope)
+    on = run()
+    assert scopes and all(scopes)
+    monkeypatch.setattr(N, "pdl_scope", lambda on: contextlib.nullcontext())
+    assert all(torch.equal(a, b) for a, b in zip(on, run()))
