@@ -70,6 +70,8 @@ def test_long_contexts_keep_one_copy():
     from zero_to_hero_b200.ops import native as N
 
     assert N.flash_bwd_copies(16, 1024, 12) == 8 and N.flash_bwd_copies(1, 65536, 16) == 1
+    assert N.flash_bwd_copies(16, 1024, 12, 384) == 8 and N.flash_bwd_copies(16, 1024, 12, 383) == 1
+    assert N.flash_bwd_copies(1, 128, 1, 0) == N.flash_bwd_copies(1, 129, 1, 0) == 1
 
 
 # fewer positions than vocabulary rows (a warp per position) and as many (a warp per row); more than one

@@ -363,6 +363,25 @@ def test_deterministic_mode_repeats_training_bit_for_bit(dropout):
     _lib.check_status()
 
 
+def test_reproducible_mode_within_a_memory_limit():
+    from zero_to_hero_b200.engine import GPT2TrainEngine
+
+    def run(limit):
+        cfg = _cfg()
+        cfg.train.deterministic = True
+        if limit is not None:
+            cfg.train.deterministic_scratch_mb = limit
+        eng = GPT2TrainEngine(cfg, "cuda", seed=3)
+        g = torch.Generator().manual_seed(5)
+        for _ in range(2):
+            eng.train_step(_batches(g), lr=1e-3)
+        return eng.dq_accum.numel(), eng.p32.clone(), eng.m.clone()
+
+    (some, *a), (none, *b), (default, *c) = run(2.0), run(0), run(None)
+    assert some == default == 2 * none  # 256 tokens: two copies of 1 MiB
+    assert all(torch.equal(x, y) and torch.equal(x, z) for x, y, z in zip(a, b, c))
+
+
 # Dependent launch moves the start of every kernel ahead of the end of the one before: what a kernel reads too
 # early shows as other bits. Reproducible sums, weight gradients on the side stream, with and without dropout.
 @pytest.mark.parametrize("dropout", (0.0, 0.2))

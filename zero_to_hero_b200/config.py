@@ -77,6 +77,9 @@ class TrainConfig:
     # order instead (split-K weight gradients folded slice by slice, attention dQ added up in KV-tile order,
     # bias and embedding gradients by ordered sums). Slower than the default.
     deterministic: bool = False
+    # Memory that mode may take for copies of attention's dQ, one per 128 keys; with less than they need (or 0) the
+    # attention backward runs one launch per 128 keys instead, slower and with the same bits.
+    deterministic_scratch_mb: float = 512.0
     log_jsonl: str = ""
 
 

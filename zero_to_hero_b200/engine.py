@@ -302,7 +302,8 @@ class GPT2TrainEngine:
             self.d_drop = [buf(M, C), buf(M, C)]
         self.d_4c = buf(M, 4 * C)
         self.d_qkv = buf(M, 3 * C)
-        self.dq_copies = N.flash_bwd_copies(B, T, H) if self.cfg.train.deterministic else 1
+        tc = self.cfg.train
+        self.dq_copies = N.flash_bwd_copies(B, T, H, tc.deterministic_scratch_mb) if tc.deterministic else 1
         self.dq_accum = buf(N.flash_bwd_dq_elems(B, T, H) * self.dq_copies, dtype=f32)
         self.attn_stats = buf(N.flash_bwd_stats_elems(B, T, H), dtype=f32)
         self.ln_scratch = buf(N.layernorm_bwd_num_partials(M) * 3 * C, dtype=f32)

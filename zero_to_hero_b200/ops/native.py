@@ -265,14 +265,11 @@ def flash_bwd_dq_elems(B: int, T: int, H: int) -> int:
     return (B * T + 31) // 32 * 32 * H * 64
 
 
-ORDERED_DQ_BYTES = 512 << 20  # memory the copies of dQ may take
-
-
-def flash_bwd_copies(B: int, T: int, H: int) -> int:
+def flash_bwd_copies(B: int, T: int, H: int, limit_mb: float = 512.0) -> int:
     """dq_accum copies worth having for the ordered form: one per 128-key tile, or 1 where they would take
-    more than ORDERED_DQ_BYTES (long contexts: their number and their size both grow with T)."""
+    more than `limit_mb` (long contexts: their number and their size both grow with T)."""
     n = (T + 127) // 128
-    return n if n * flash_bwd_dq_elems(B, T, H) * 4 <= ORDERED_DQ_BYTES else 1
+    return n if n * flash_bwd_dq_elems(B, T, H) * 4 <= limit_mb * 2 ** 20 else 1
 
 
 def flash_bwd(qkv, out, dout, lse, dqkv, dq_accum, stats, B, T, H, drop_p: float = 0.0, seed=None,
