@@ -58,7 +58,7 @@ def _grads(model, X, Y):
     model.zero_grad(set_to_none=True)
     logits, loss = model(X, Y)
     loss.backward()
-    return logits.detach().double().cpu(), [p.grad.double().cpu() for p in model.parameters()]
+    return logits.detach().double().cpu(), [p.grad.double().cpu() for p in model.parameters()], float(loss.detach())
 
 
 # one token, a whole and a part of a 32-row group, several tiles; one head up to a wide block; tied and untied
@@ -93,6 +93,21 @@ def test_block_matches_the_single_ops(make, B, T, kw, bf16):
     # the same rounding points, so two draws of one error; 2e-3 is a single bf16 rounding
     for a, b in zip(off(got), off(single)):
         assert a <= 1.3 * b + 2e-3, (off(got), off(single))
+    # each parameter by itself, as errors in a bias or LayerNorm gradient do not show beside the matrices (the two
+    # are within 1.2 of each other; what is a thousandth of all gradients together is noise)
+    whole = torch.sqrt(sum(v.square().sum() for v in ref[1]))
+    for (n, _), r, a, b in zip(m.named_parameters(), ref[1], got[1], single[1]):
+        assert (a - r).norm() <= 1.3 * (b - r).norm() + 2e-3 * max(r.norm(), 1e-3 * whole), n
+    # the loss: that of the logits beside it, and off from the exact one by the mean of the tokens' errors, which
+    # is their size over sqrt(tokens), and by the second-order term of the logits' errors
+    def per_token(logits):
+        return nn.functional.cross_entropy(logits.flatten(0, 1), Y.flatten(), reduction="none")
+
+    for r in (got, single):
+        assert abs(r[2] - float(per_token(r[0]).mean())) < 1e-5 * abs(r[2])
+        d = per_token(r[0]) - per_token(ref[0])
+        assert abs(r[2] - ref[2]) <= 4 * float(d.square().mean().sqrt()) / d.numel() ** 0.5 + \
+            float((r[0] - ref[0]).square().mean())
     frozen = [p for b in blocks for p in b.parameters() if p.dim() >= 2][:2]
     for p in frozen:
         p.requires_grad_(False)
