@@ -54,6 +54,44 @@ def test_only_plain_blocks_are_fused():
         assert FB.shaped([None if j == i else t for j, t in enumerate(whole)], shapes) == (i in (1, 2, 4, 6, 8, 10))
 
 
+def test_blocks_with_replaced_parts_are_not_touched():
+    class Odd(nn.Module):  # none of the attributes of what it stands for
+        def forward(self, *args):
+            return args[0]
+
+    def gone(make, path):
+        m = make()
+        b = m.transformer.h[0] if make is _gpt2 else m.blocks[0]
+        *way, last = path.split(".")
+        owner = b
+        for name in way:
+            owner = getattr(owner, name)
+        setattr(owner, last, Odd())
+        return b._parts()
+
+    for path in ("ln_1", "ln_2", "attn", "mlp", "attn.c_attn", "attn.c_proj", "mlp.c_fc", "mlp.c_proj"):
+        assert gone(_gpt2, path) is None, path
+    for path in ("ln1", "ln2", "attn", "ff", "attn.proj", "attn.heads", "ff.ff", "attn.heads.0", "attn.heads.1.key",
+                 "ff.ff.0", "ff.ff.1", "ff.ff.2", "ff.ff.4"):
+        assert gone(_char, path) is None, path
+
+
+# the same on a GPU: such a block runs through its parts
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", (_gpt2, _char))
+def test_block_with_another_attention_runs(make):
+    class Own(nn.Module):
+        def forward(self, x, residual=None, cdrop=None):
+            return x if residual is None else residual + x
+
+    m = make()
+    (m.transformer.h[0] if make is _gpt2 else m.blocks[0]).attn = Own()
+    m = m.cuda()
+    X = torch.randint(0, 60, (2, 9)).cuda()
+    m(X, X)[1].backward()
+    assert all(p.grad.isfinite().all() for p in m.parameters())
+
+
 def _grads(model, X, Y):
     model.zero_grad(set_to_none=True)
     logits, loss = model(X, Y)

@@ -108,16 +108,19 @@ class Block(nn.Module):
         """(parameters of `ops.block.block`) when calling the parts of this block would run exactly their
         classes' forwards without dropout, else None."""
         attn, ff = self.attn, self.ff
-        seq = ff.ff
-        known = [(self.ln1, LayerNorm), (self.ln2, LayerNorm), (attn, MultiHeadAttention), (attn.proj, nn.Linear),
-                 (attn.heads, nn.ModuleList), (ff, FeedForward), (seq, nn.Sequential)]
-        if len(seq) != 5 or len(attn.heads) != attn.num_heads:
+        # what a replaced part has is known only once it is one of these: each level before the next is touched
+        if type(attn) is not MultiHeadAttention or type(ff) is not FeedForward or (attn.training and attn.p > 0.0):
             return None
+        seq, heads = ff.ff, attn.heads
+        if type(seq) is not nn.Sequential or type(heads) is not nn.ModuleList or len(seq) != 5 or \
+                len(heads) != attn.num_heads or any(type(h) is not Head for h in heads):
+            return None
+        known = [(self.ln1, LayerNorm), (self.ln2, LayerNorm), (attn, MultiHeadAttention), (attn.proj, nn.Linear),
+                 (heads, nn.ModuleList), (ff, FeedForward), (seq, nn.Sequential)]
         known += list(zip(seq, (nn.Linear, nn.ReLU, nn.Dropout, nn.Linear, nn.Dropout)))
-        known += [(h, Head) for h in attn.heads]
-        known += [(m, nn.Linear) for h in attn.heads for m in (h.query, h.key, h.value)]
-        if not plain_modules(known) or (attn.training and attn.p > 0.0) or \
-                any(d.training and d.p > 0.0 for d in (seq[2], seq[4])):
+        known += [(h, Head) for h in heads]
+        known += [(m, nn.Linear) for h in heads for m in (h.query, h.key, h.value)]
+        if not plain_modules(known) or any(d.training and d.p > 0.0 for d in (seq[2], seq[4])):
             return None
         if any(m.bias is not None for h in attn.heads for m in (h.query, h.key, h.value)):
             return None

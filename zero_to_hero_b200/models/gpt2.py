@@ -114,9 +114,13 @@ class Block(nn.Module):
         """(parameters of `ops.block.block`) when calling the parts of this block would run exactly their
         classes' forwards without dropout, else None."""
         attn, mlp = self.attn, self.mlp
+        # what a replaced part has is known only once it is one of these
+        if type(attn) is not Attention or type(mlp) is not MLP or (attn.training and attn.dropout > 0.0) or \
+                (mlp.training and mlp.dropout > 0.0):
+            return None
         known = ((self.ln_1, LayerNorm), (self.ln_2, LayerNorm), (attn, Attention), (mlp, MLP), (attn.c_attn, nn.Linear),
                  (attn.c_proj, nn.Linear), (mlp.c_fc, nn.Linear), (mlp.c_proj, nn.Linear))
-        if not plain_modules(known) or (attn.training and attn.dropout > 0.0) or (mlp.training and mlp.dropout > 0.0):
+        if not plain_modules(known):
             return None
         return ((self.ln_1.weight, self.ln_1.bias), attn.c_attn.bias, (attn.c_proj.weight, attn.c_proj.bias),
                 (self.ln_2.weight, self.ln_2.bias), (mlp.c_fc.weight, mlp.c_fc.bias),
