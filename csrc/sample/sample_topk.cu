@@ -217,12 +217,7 @@ int sample_topk(const float* logits, long long* out, long long out_stride, int B
 
 }  // namespace z2h
 
-extern "C" int z2h_sample_topk(const float* logits, long long* out, int B, int V, long long ld,
-                               float temperature, int top_k, unsigned long long seed,
-                               unsigned long long offset, void* stream) {
-  return z2h::sample_topk(logits, out, 1, B, V, ld, temperature, top_k, seed, offset, (cudaStream_t)stream);
-}
-// The same with the id of row b written to out[b * out_stride].
+// The id of row b is written to out[b * out_stride].
 extern "C" int z2h_sample_topk_strided(const float* logits, long long* out, long long out_stride, int B, int V,
                                        long long ld, float temperature, int top_k, unsigned long long seed,
                                        unsigned long long offset, void* stream) {
