@@ -227,7 +227,7 @@ def test_generate_raises_what_a_kernel_reported():
 # the top-k select: values that crowd into one first digit, ties, both signs of zero, -inf, one row in
 # shared memory and one too long for it
 @pytest.mark.gpu
-@pytest.mark.parametrize("V", (1, 33, 1000, 50257, 56321))
+@pytest.mark.parametrize("V", (1, 33, 1000, 50257, 56320, 56321))
 def test_top_k_keeps_what_the_sort_keeps(V):
     from zero_to_hero_b200.ops.sampling import sample_next, sample_topk_native
 
