@@ -31,10 +31,10 @@
 //
 // By-product: the column sums of dK and dV (this kernel's epilogue) and of dQ (the conversion kernel)
 // can be added to an fp32 vector, which is the gradient of the QKV projection's bias.
-// Reproducible form (flash_bwd_ex, ordered): every KV tile stores its dQ contributions to a copy of the
-// buffer of its own and the conversion kernel adds the copies in KV-tile order: one launch that fills the
-// SMs instead of one per KV tile (5 x 509 tokens, 6 heads: 14.7 us instead of 4 x 11.9). Where the caller
-// has only one copy's memory, one launch per KV tile, so that the additions happen in the same order.
+// Reproducible form (ordered): with a copy of the dQ buffer per KV tile (flash_bwd_sliced) every tile stores its
+// contributions to its own and the conversion kernel adds the copies in KV-tile order: one launch that fills the
+// SMs instead of one per KV tile (5 x 509 tokens, 6 heads: 14.7 us instead of 4 x 11.9). With one copy's memory
+// (flash_bwd_ex, or fewer copies), one launch per KV tile, so that the additions happen in the same order.
 //
 // This is the hand-written counterpart of what autograd runs for
 // F.scaled_dot_product_attention in the reference (nn/gpt2/modules.py:37, train_ddp.py:141).

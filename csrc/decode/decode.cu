@@ -79,7 +79,7 @@ __host__ __device__ inline Cut cut_matrix(int slot_bytes, int n, int K, int grid
 }
 
 // What a CTA does, worked out once per launch: integer divisions inside the phases cost more than their
-// arithmetic (about 2,000 cycles a phase, measured).
+// arithmetic.
 enum Matrix : int { kQkv, kProj, kFc, kFc2, kHead, kMatrices };
 struct Share {
   int r0, r1;      // its rows of a matrix, a run that starts on an even row
@@ -588,9 +588,8 @@ __device__ __forceinline__ void fold_attention(const Params& p, Smem* sm, uint8_
 }
 
 // One loop over the phases of all layers with a single instance of each piece of code: laid out phase by
-// phase the kernel was 170 KB of code (65 KB now) and every phase began with instruction-cache misses (one
-// token of the 124M model 330 us, 230 so; of the 1.5B model for four sequences 2.4 and 1.65 ms). The bounded
-// waits are inlined all the same: out of line each cost some 500 cycles.
+// phase, the same code took 330 us for one token of the 124M model instead of 230 and 2.4 ms instead of 1.65 for
+// one of the 1.5B model in four sequences. The bounded waits are inlined all the same.
 __device__ __forceinline__ void consume(const Params& p, Smem* sm, const uint8_t* ring, uint8_t* xs) {
   const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(p.a.weights);
   const DecodeLayout& lay = p.a.lay;

@@ -4,15 +4,17 @@
 // One persistent CTA per SM walks a static tile schedule (M fastest, so the CTAs that run at
 // the same time share one B panel out of L2). Inside the CTA the work is split by warp role:
 //
-//   warp 0      TMA producer   cp.async.bulk.tensor 2-D tiles, 128-byte swizzle, 4-stage ring
-//   warp 1      MMA issuer     one elected lane issues tcgen05.mma (128x256x16) and commits
+//   warp 0      TMA producer   cp.async.bulk.tensor 2-D tiles, 128-byte swizzle, ring of 4 stages (6 and 8
+//                              for tiles of 128 and 64 columns)
+//   warp 1      MMA issuer     one elected lane issues tcgen05.mma (128 x BN x 16) and commits
 //                              stage releases / accumulator completions to mbarriers
-//   warps 2-9   epilogue       tcgen05.ld the 128x256 fp32 accumulator (one row per thread, two
-//                              warps per TMEM lane quarter, each taking half of the columns),
-//                              apply bias / GELU / residual / GELU' and store
+//   warps 2-9   epilogue       tcgen05.ld the 128 x BN fp32 accumulator (one row per thread, two
+//                              warps per TMEM lane quarter, each taking half of the columns; tiles of
+//                              64 columns have one per quarter, warps 2-5), apply bias / GELU / residual /
+//                              GELU' and store
 //
-// Two accumulators of 256 TMEM columns each are used in turn, so the epilogue of tile i runs
-// while the tensor cores already work on tile i+1.
+// The tile is 128 x BN, BN = 256, 128 or 64. Two accumulators of BN TMEM columns each are used in turn, so the
+// epilogue of tile i runs while the tensor cores already work on tile i+1.
 //
 // Either operand may be K-major (the contraction index is contiguous in global memory) or
 // MN-major (the M / N index is contiguous); the second form is what the weight-gradient and

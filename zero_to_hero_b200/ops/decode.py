@@ -14,7 +14,11 @@ import torch.nn as nn
 from . import _lib, gemm as G, native as N
 
 MAX_BATCH = 8            # sequences of one decode launch (the n of its tensor-core instruction)
-MAX_SEQUENCES = 32       # sequences of a session, in groups of MAX_BATCH
+# Sequences of a session, in groups of MAX_BATCH that each read all weights; more take the batched forward per
+# token, whose time hardly depends on their number while the window is short. Session / forward, ms for 8 tokens,
+# prompts of 8: 24 sequences 10.7 / 17.7 (124M) and 65 / 64 (1.5B), 32 14.0 / 17.7 and 85 / 64, 48 20.5 / 17.9 and
+# 126 / 65; prompts of 256: 32 15.3 / 22.3 and 110 / 229, 48 22.5 / 26.4 and 162 / 325.
+MAX_SEQUENCES = 32
 # A prompt of up to this many tokens (before its last one) goes through the decode kernel one by one, a longer
 # one through the batched pass, which is bound by its launches. Stepwise / batched, ms: 124M, one sequence, 4
 # tokens 0.74 / 1.09, 6 tokens 1.11 / 1.08; eight sequences, 4 tokens 1.02 / 1.08; 1.5B, 4 tokens 4.4 / 5.0,
@@ -269,6 +273,8 @@ def generate(model, X: torch.Tensor, max_new_tokens: int, temperature: float, to
         sample_next(logits, temperature, top_k, generator, out=tokens[:, T])
     if not torch.cuda.is_current_stream_capturing():
         # A wait between CTAs that ran out leaves the step's results wrong and says so in the status word alone. Read
-        # once a call, after the last launch: raises, as the engine does when it reads a loss.
+        # once a call, after the last launch: raises, as the engine does when it reads a loss. A caller that reads the
+        # tokens waits here instead of there; one that goes on launching loses that overlap (15.4 -> 16.7 ms for 64
+        # tokens of the 124M model and a forward pass).
         _lib.check_status(session.device)
     return torch.cat((X, tokens[:, T0:]), dim=1)
