@@ -397,8 +397,8 @@ class _CrossEntropySaved(torch.autograd.Function):
     """The same over bf16 logits whose rows are tight in memory, any vocabulary: one pass forward that keeps
     a copy of the logits (the caller's may change before the backward), one pass backward that rounds the
     gradient once. The copy is an output beside the loss: saved like any tensor and freed with the graph, and
-    what a second derivative goes through. `skip_ignored`: the mean is over the targets that are not ignored, and a label that names
-    neither a class nor -100 makes it NaN (and shows in the status word)."""
+    what a second derivative goes through. `skip_ignored`: the mean is over the targets that are not ignored,
+    and a label that names neither a class nor -100 makes it NaN (and shows in the status word)."""
 
     @staticmethod
     def forward(ctx, logits, targets, v_real, skip_ignored):
