@@ -49,3 +49,20 @@ def test_traces_and_transforms_are_seen():
     assert len(seen) == 7 and all(seen[1:])
     look(x)
     assert not seen[-1]
+
+
+def test_tensors_of_another_device_than_the_current_one(monkeypatch):
+    class On:
+        def __init__(self, device):
+            self.device = torch.device(device)
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    assert Z._here(On("cuda:1")) and not Z._here(On("cuda:0")) and not Z._here(On("cuda:2"))
+    # as on a GPU, on another device: the library's operations
+    monkeypatch.setattr(Z, "_native", lambda t: True)
+    monkeypatch.setattr(Z, "_here", lambda t: False)
+    g = torch.Generator().manual_seed(1)
+    x, w = torch.randn(4, 16, generator=g).bfloat16(), torch.randn(7, 16, generator=g).bfloat16()
+    logits, targets = Z.linear(x, w), torch.tensor([0, 6, -100, 3])
+    assert torch.equal(logits, torch.nn.functional.linear(x, w))
+    assert torch.equal(Z.cross_entropy(logits, targets), torch.nn.functional.cross_entropy(logits.float(), targets))

@@ -152,6 +152,11 @@ def _transformed() -> bool:
     return torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0
 
 
+def _here(t: torch.Tensor) -> bool:
+    """On the current device, where launches go; the library's operations run where their tensors are."""
+    return t.device.index is None or t.device.index == torch.cuda.current_device()
+
+
 def _any_width_ok(x, w, b) -> bool:
     """Whether `_LinearAnyWidth` computes what F.linear over bf16 casts does here. Anything that F.linear refuses,
     broadcasts or computes in another type or order goes to it: the kernels take plain addresses."""
@@ -159,7 +164,7 @@ def _any_width_ok(x, w, b) -> bool:
         return False
     if b is not None and b.shape != w.shape[:1]:
         return False
-    if any(t.device != x.device for t in (w, b) if t is not None):
+    if not _here(x) or any(t.device != x.device for t in (w, b) if t is not None):
         return False
     if torch.is_autocast_enabled(x.device.type) and torch.get_autocast_dtype(x.device.type) != torch.bfloat16:
         return False
@@ -453,7 +458,7 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, v_real: int | Non
             if tight and t.dtype in (torch.int64, torch.int32):
                 return _CrossEntropySaved.apply(x, t, v_real, False)[0]
             return _CrossEntropy.apply(x, t, v_real)
-        if tight and t.dtype == torch.int64 and t.device == x.device and not _transformed():
+        if tight and t.dtype == torch.int64 and t.device == x.device and _here(x) and not _transformed():
             return _CrossEntropySaved.apply(x, t, v_real, True)[0]
     if _native(logits):
         FALLBACK_COUNTS["cross_entropy"] += 1
